@@ -12,6 +12,15 @@ namespace lc {
 // ---------------------------------------------------------------------------
 // geometry
 // ---------------------------------------------------------------------------
+// one point of every pair of opposite lattice points
+static void set_lattice(PolarPts &p, int lat) {
+    p.lat = lat;
+    p.half = (lat + 1) / 2;
+    p.M = (long)p.ntheta * lat;
+    p.Mh = (long)p.ntheta * p.half;
+    p.div_angle = make_fastdiv((unsigned)p.half);
+}
+
 void geometry_init_2d(Context &ctx, PolarGeometry &g, const double *theta, int ntheta, int nr) {
     LC_REQUIRE(ntheta > 0 && nr > 0, "geometry: ntheta and nradial must be positive");
     LC_REQUIRE((long)ntheta * nr < (1L << 31), "geometry: too many points");
@@ -24,9 +33,8 @@ void geometry_init_2d(Context &ctx, PolarGeometry &g, const double *theta, int n
     g.pts.dim = 2;
     g.pts.ntheta = ntheta;
     g.pts.nr = nr;
-    g.pts.M = (long)ntheta * nr;
     g.pts.cs = g.cs.get();
-    g.pts.div_angle = make_fastdiv((unsigned)nr);
+    set_lattice(g.pts, nr);
 }
 
 void geometry_init_3d(Context &ctx, PolarGeometry &g, const double *theta, const double *gamma,
@@ -60,9 +68,8 @@ void geometry_init_3d(Context &ctx, PolarGeometry &g, const double *theta, const
     g.pts.ntheta = ntheta;
     g.pts.nrows = nrows;
     g.pts.ncols = ncols;
-    g.pts.M = (long)ntheta * nrows * ncols;
     g.pts.rot = g.rot.get();
-    g.pts.div_angle = make_fastdiv((unsigned)nrows * (unsigned)ncols);
+    set_lattice(g.pts, nrows * ncols);
     g.pts.div_col = make_fastdiv((unsigned)ncols);
 }
 
@@ -142,27 +149,26 @@ __device__ __forceinline__ unsigned fast_div(unsigned n, FastDiv f) { return (__
 struct PointInfo {
     double c[3];  // x, y, z
     double qX, qY;
-    int angle;
+    int angle, l;  // angle and lattice point
+    bool flip;     // c is the negated coordinate
 };
 
-__device__ __forceinline__ void point_at(const PolarPts &p, long j, PointInfo &pi) {
-    const unsigned jj = (unsigned)j;  // M < 2^31
+// lattice point l of angle i
+__device__ __forceinline__ void lattice_point(const PolarPts &p, int i, int l, PointInfo &pi) {
+    pi.angle = i;
+    pi.l = l;
+    pi.flip = false;
     if (p.dim == 2) {
-        const int i = (int)fast_div(jj, p.div_angle);
-        const int m = (int)(jj - (unsigned)i * (unsigned)p.nr);
-        double r = ((double)m + 0.5) * (2.0 * kPi / p.nr) - kPi;
+        double r = ((double)l + 0.5) * (2.0 * kPi / p.nr) - kPi;
         double2 cs = p.cs[i];
         pi.c[0] = cs.x * r;
         pi.c[1] = cs.y * r;
         pi.c[2] = 0.0;
-        pi.angle = i;
         pi.qX = r;
         pi.qY = 0.0;
     } else {
-        const unsigned i = fast_div(jj, p.div_angle);
-        const unsigned rem = jj - i * ((unsigned)p.nrows * (unsigned)p.ncols);
-        const unsigned ua = fast_div(rem, p.div_col);
-        const int a = (int)ua, b = (int)(rem - ua * (unsigned)p.ncols);
+        const unsigned ua = fast_div((unsigned)l, p.div_col);
+        const int a = (int)ua, b = l - (int)ua * p.ncols;
         double qX = ((double)b + 0.5) * (2.0 * kPi / p.ncols) - kPi;
         double qY = ((double)a + 0.5) * (2.0 * kPi / p.nrows) - kPi;
         const double *R = p.rot + 6 * (long)i;
@@ -171,12 +177,51 @@ __device__ __forceinline__ void point_at(const PolarPts &p, long j, PointInfo &p
         pi.c[2] = R[4] * qX + R[5] * qY;
         pi.qX = qX;
         pi.qY = qY;
-        pi.angle = (int)i;
+    }
+}
+
+// Folded point j: one of each pair of opposite lattice points, negated when
+// its y coordinate (wrapped to [-pi, pi]) is below zero, so that the folded
+// points fill the half of the fine grid with y >= 0 at the density of the
+// full set.
+__device__ __forceinline__ void point_at(const PolarPts &p, long j, PointInfo &pi) {
+    const unsigned jj = (unsigned)j;  // below 2^31
+    const unsigned i = fast_div(jj, p.div_angle);
+    lattice_point(p, (int)i, (int)(jj - i * (unsigned)p.half), pi);
+    if (pi.c[1] - 2.0 * kPi * rint(pi.c[1] * kInv2Pi) < 0.0) {
+        pi.flip = true;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) pi.c[d] = -pi.c[d];
     }
 }
 
 __device__ __forceinline__ bool in_band(const PointInfo &pi) {
     return fabs(pi.c[0]) <= kPi && fabs(pi.c[1]) <= kPi && fabs(pi.c[2]) <= kPi;
+}
+
+// Band flags kept in the upper bits of a sorted point's corner: the point and
+// its opposite are tested separately (rounding decides for a lattice point on
+// the boundary).
+constexpr unsigned kCornerMask = 0x3fffu, kOutOwn = 0x8000u, kOutOpp = 0x4000u;
+
+// Type 1 keeps the real part of sum_j c_j exp(i k.x_j).  The pair x, -x adds
+//   Re(c e^{i k.x} + c' e^{-i k.x}) = Re((c + conj c') e^{i k.x}),
+// so one point with the value c + conj(c') stands for both (its conjugate
+// when the point is negated), at half the footprints to spread: the 3D
+// spreading of 360 x 511 x 511 values onto 48 x 1024 x 1024 cells took 14.3 ms
+// with every point and 7.1 ms folded.  Values outside the band are left out; cv is the volume's value array, out the flags
+// that count.
+__device__ __forceinline__ float2 fold_value(const PolarPts &p, const float2 *__restrict__ cv, int angle, int l,
+                                             unsigned out) {
+    const float2 *a = cv + (long)angle * p.lat;
+    float2 v = make_float2(0.f, 0.f);
+    if (!(out & kOutOwn)) v = a[l];
+    if (2 * l + 1 != p.lat && !(out & kOutOpp)) {
+        const float2 w = a[p.lat - 1 - l];
+        v.x += w.x;
+        v.y -= w.y;
+    }
+    return v;
 }
 
 // wrapped fine-grid coordinate u in [0, nf), its cell, first covered cell l0
@@ -232,7 +277,7 @@ __device__ __forceinline__ int bin_of(const PointInfo &pi, const GridCfg &g, int
 
 template <int DIM>
 __global__ void bin_count_kernel(PolarPts pts, GridCfg g, int W, int *counts) {
-    for (long j = (long)blockIdx.x * blockDim.x + threadIdx.x; j < pts.M;
+    for (long j = (long)blockIdx.x * blockDim.x + threadIdx.x; j < pts.Mh;
          j += (long)gridDim.x * blockDim.x) {
         PointInfo pi;
         point_at(pts, j, pi);
@@ -265,18 +310,24 @@ __device__ __forceinline__ int bin_corner_of(const PointInfo &pi, const GridCfg 
     return b;
 }
 
-// perm[k] = the point at sorted position k; corners[k] its footprint corner
-// in its bin's tile (read by the footprint bound and the spreading's
-// bucketing)
+// perm[k] = the folded point at sorted position k; corners[k] its footprint
+// corner in its bin's tile (read by the footprint bound and the spreading's
+// bucketing) and its band flags
 template <int DIM>
 __global__ void bin_scatter_kernel(PolarPts pts, GridCfg g, int W, int *cursor, int *perm,
                                    unsigned short *corners) {
-    for (long j = (long)blockIdx.x * blockDim.x + threadIdx.x; j < pts.M;
+    for (long j = (long)blockIdx.x * blockDim.x + threadIdx.x; j < pts.Mh;
          j += (long)gridDim.x * blockDim.x) {
         PointInfo pi;
         point_at(pts, j, pi);
         int corner;
         int b = bin_corner_of<DIM>(pi, g, W, corner);
+        if (DIM == 3) {
+            if (!in_band(pi)) corner |= (int)kOutOwn;
+            PointInfo po;
+            lattice_point(pts, pi.angle, pts.lat - 1 - pi.l, po);
+            if (!in_band(po)) corner |= (int)kOutOpp;
+        }
         unsigned act = __activemask();
         unsigned peers = __match_any_sync(act, b);
         int lane = threadIdx.x & 31;
@@ -308,7 +359,14 @@ __global__ void bin_scatter_kernel(PolarPts pts, GridCfg g, int W, int *cursor, 
 //     plane stride; the rotation fits when both banks of every point of the
 //     high round are clear of the low round's banks.  The pairing depends on
 //     the bank counts alone, so every warp walks it and spreads the passes
-//     that fall to it.  (2D tiles run the tail rounds one by one.)
+//     that fall to it.
+//   * tail rounds, 2D: packed, 32 points to a pass, in the order of the rounds.
+//     A pass over rounds of k banks has conflicts of degree 32 / k, the same
+//     shared-memory cycles as its rounds one by one, but a point's latency
+//     (its value's load, the 64-bit placement, the weights) is paid once for
+//     32 points.  The bins around the origin hold hundreds of points on a few
+//     banks; their serial rounds set the kernel's time (four 1023^2 slices,
+//     720 angles: 0.26 ms with serial rounds, 0.14 ms packed).
 // The accumulation is exact and order-free (below): the schedule decides the
 // speed, never the result.
 //
@@ -328,14 +386,14 @@ __global__ void bin_scatter_kernel(PolarPts pts, GridCfg g, int W, int *cursor, 
 // 1.5 * 2^23, which places it in the low mantissa bits (|v F_b| < 2^22), and
 // the float's bits are added as they are: every contribution then carries
 // the bias 0x4B400000, and the flush subtracts K_cell times it (modulo 2^32)
-// with K_cell the footprints over the cell.  With F_b m_b <= 2^21 and
-// K_b m_b F_b < 2^30 a tile cell's sum stays below 2^31, so the word holds it
+// with K_cell the footprints over the cell.  With F_b m_b < 2^22 and
+// W_b m_b F_b < 2^31 a tile cell's sum stays below 2^31, so the word holds it
 // exactly.  The flush adds each sum, shifted to one scale F_G = 2^e_G for
 // the whole launch (e_b <= e_G, so the shift is exact), to a 64-bit integer
 // per part of the fine grid, and a conversion pass forms the float grid.
 // Every sum is an exact integer, so the fine grid depends neither on the
 // order of the atomics nor on the schedule: a backprojection is bit-for-bit
-// repeatable.  The rounding step 1 / F_b is at most max(W_b 2^-29, 2^-20) m_b:
+// repeatable.  The rounding step 1 / F_b is at most max(W_b 2^-30, 2^-21) m_b:
 // a cell summed from K footprints is within about sqrt(K / 12) of that of its
 // exact value.
 constexpr int kSpreadThreads = 256;
@@ -345,10 +403,11 @@ constexpr unsigned kRoundMagicBits = 0x4B400000u;
 // Exponents of the fixed-point scales.  Launch: F_G = 2^e_G with
 // kmax m F_G < 2^61 (kmax bounds the footprints over one fine-grid cell, m
 // the values), so a cell's 64-bit sum stays below 2^62.  Bin: F_b = 2^e_b
-// with F_b m_b <= 2^21 (rounding by 1.5 2^23) and W_b m_b F_b < 2^30, W_b a
-// bound on the sum of the weights of the bin's footprints over one cell, so
-// a tile cell's sum (plus at most 1024 rounding halves) stays below 2^31;
-// and e_b <= e_G.
+// with F_b m_b < 2^22 (rounding by 1.5 2^23) and W_b m_b F_b < 2^31, W_b a
+// bound on the sum of the weights of the bin's footprints over one cell.  W_b
+// exceeds the largest sum by its margins of 1e-3 per axis and 1e-4, above
+// 2^20 steps of a sum near 2^31, so the sum and its at most 1024 rounding
+// halves stay below 2^31; and e_b <= e_G.
 __host__ __device__ __forceinline__ int fix_exponent_grid(float m, long kmax) {
     if (!(m > 0.f)) return 0;
     int e3;
@@ -360,22 +419,9 @@ __device__ __forceinline__ int fix_exponent_tile(float mb, float wb, int eg) {
     int e1, e2;
     frexp((double)mb, &e1);               // m_b < 2^e1
     frexp((double)wb * (double)mb, &e2);  // W_b m_b < 2^e2
-    const int a = 21 - e1, b = 30 - e2;
+    const int a = 22 - e1, b = 31 - e2;
     const int e = a < b ? a : b;
     return e < eg ? e : eg;
-}
-
-// m = max |Re c| + |Im c| over n values, as the bits of a non-negative float
-// (integer order equals float order); *bits must start at 0
-__global__ void value_bound_kernel(const float2 *__restrict__ c, long n, int *bits) {
-    float m = 0.f;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const float2 v = c[i];
-        m = fmaxf(m, fabsf(v.x) + fabsf(v.y));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(bits, __float_as_int(m));
 }
 
 // fine grid <- T / F_G from the two 64-bit fixed-point sums per cell
@@ -456,12 +502,12 @@ __device__ __forceinline__ void rot_banks(int rot, int plane, int &d1, int &d2) 
     d2 = (plane * (rot - W)) & 31;
 }
 
-// Spreads point j; in 3D its footprint planes are visited in the order rotated
+// Spreads the folded point j (cf: its corner and band flags); in 3D its footprint planes are visited in the order rotated
 // by rot (0: in order).
 template <int DIM, int W>
 __device__ __forceinline__ void spread_point(const PolarPts &pts, const GridCfg &g,
-                                             const float2 *__restrict__ c, long cstride, int nvol, int j,
-                                             int mode, const float2 *__restrict__ shifts, const int (&S)[3],
+                                             const float2 *__restrict__ c, int nvol, int j, unsigned cf,
+                                             int mode, const float2 *__restrict__ shifts,
                                              int tx, int plane, int tsize, unsigned sm_re,
                                              unsigned plane_bytes, float fscale, int rot) {
     const float inv_hw = 2.0f / (float)W;
@@ -477,15 +523,14 @@ __device__ __forceinline__ void spread_point(const PolarPts &pts, const GridCfg 
     }
     // wk[d][m]: weight of the cell at offset m along axis d (3D z: (m + rot) mod W)
     float wk[DIM][W];
-    int corner = 0;
+    const int corner = (int)(cf & kCornerMask);
+    const unsigned out = mode == PT_PLAIN ? 0u : cf;
     {
-        const int stride[3] = {1, tx, plane};
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
             int cell, l0;
             float off;
             place(pi.c[d], g.nf[d], g.inv_nf[d], W, cell, l0, off);
-            corner += (l0 - S[d]) * stride[d];
             const int r = d == 2 ? rot : 0;
 #pragma unroll
             for (int m = 0; m < W; ++m) {
@@ -496,8 +541,9 @@ __device__ __forceinline__ void spread_point(const PolarPts &pts, const GridCfg 
         }
     }
     for (int s = 0; s < nvol; ++s) {
-        float2 v = c[(long)s * cstride + j];
+        float2 v = fold_value(pts, c + (long)s * pts.M, pi.angle, pi.l, out);
         v = mode == PT_SHIFT ? cmul(v, mult) : make_float2(v.x * fscale, v.y * fscale);
+        if (pi.flip) v.y = -v.y;
         // 32-bit shared addresses of the footprint corner in the two planes
         const unsigned ar = sm_re + 4u * (unsigned)(s * tsize + corner);
         const unsigned ai = ar + plane_bytes;
@@ -557,7 +603,7 @@ __global__ void __launch_bounds__(256) bin_footprint_kernel(GridCfg g, OffsetWei
     for (int i = threadIdx.x; i < tsize; i += blockDim.x) hist[i] = 0;
     if (threadIdx.x == 0) kmx = 0;
     __syncthreads();
-    for (int p = threadIdx.x; p < br.y; p += blockDim.x) atomicAdd(&hist[corners[br.x + p]], 1);
+    for (int p = threadIdx.x; p < br.y; p += blockDim.x) atomicAdd(&hist[corners[br.x + p] & kCornerMask], 1);
     __syncthreads();
     // weighted sums along x, y, z in place, one thread per line with the
     // last W inputs in registers
@@ -596,23 +642,37 @@ __global__ void __launch_bounds__(256) bin_footprint_kernel(GridCfg g, OffsetWei
     if (threadIdx.x == 0) kbin[blockIdx.x] = __float_as_int(__int_as_float(kmx) * 1.0001f);
 }
 
-// Per launch: m_b of every bin (float bits, binm zeroed first) over all
-// values of the bin's points (one CTA per subproblem)
-__global__ void __launch_bounds__(256) bin_value_bound_kernel(const float2 *__restrict__ c, long cstride,
+// Per call: m_b = max |Re v| + |Im v| of every bin over the folded values v of
+// the bin's points (one CTA per subproblem), and their maximum over the launch,
+// as the bits of non-negative floats (integer order equals float order; binm
+// and mbits zeroed first)
+__global__ void __launch_bounds__(256) bin_value_bound_kernel(PolarPts pts, const float2 *__restrict__ c,
                                                               int nvol, const int *__restrict__ perm,
-                                                              const int4 *__restrict__ subs, int *binm) {
+                                                              const unsigned short *__restrict__ corners,
+                                                              const int4 *__restrict__ subs, int mode, int *binm,
+                                                              int *mbits) {
+    __shared__ int mx;
     const int4 sp = subs[blockIdx.x];
+    if (threadIdx.x == 0) mx = 0;
+    __syncthreads();
     float m = 0.f;
     for (int p = threadIdx.x; p < sp.z; p += blockDim.x) {
-        const int j = perm[sp.y + p];
+        const unsigned j = (unsigned)perm[sp.y + p];
+        const unsigned i = fast_div(j, pts.div_angle);
+        const unsigned out = mode == PT_PLAIN ? 0u : corners[sp.y + p];
         for (int s = 0; s < nvol; ++s) {
-            const float2 v = c[(long)s * cstride + j];
+            const float2 v = fold_value(pts, c + (long)s * pts.M, (int)i, (int)(j - i * (unsigned)pts.half), out);
             m = fmaxf(m, fabsf(v.x) + fabsf(v.y));
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(&binm[sp.x], __float_as_int(m));
+    if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(&mx, __float_as_int(m));
+    __syncthreads();
+    if (threadIdx.x == 0 && mx > 0) {
+        atomicMax(&binm[sp.x], mx);
+        atomicMax(mbits, mx);
+    }
 }
 
 #ifndef LC_SPREAD_MIN_BLOCKS
@@ -621,7 +681,7 @@ __global__ void __launch_bounds__(256) bin_value_bound_kernel(const float2 *__re
 
 template <int DIM, int W>
 __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
-    spread_kernel(PolarPts pts, GridCfg g, const float2 *__restrict__ c, long cstride, int nvol,
+    spread_kernel(PolarPts pts, GridCfg g, const float2 *__restrict__ c, int nvol,
                   const int *__restrict__ perm, const unsigned short *__restrict__ corners,
                   const int4 *__restrict__ subs,
                   unsigned long long *__restrict__ fix, long gstride, int mode,
@@ -663,15 +723,10 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
         const int p = tid + q * (int)blockDim.x;
         key[q] = -1;
         if (p >= sp.z) continue;
-        bool use = true;
-        if (mode != PT_PLAIN) {
-            PointInfo pi;
-            point_at(pts, perm[sp.y + p], pi);
-            use = in_band(pi);
-        }
         int k = -1;
-        if (use) {
-            const int corner = corners[sp.y + p];  // from the bin sort
+        const unsigned cf = corners[sp.y + p];  // from the bin sort
+        if (mode == PT_PLAIN || (cf & (kOutOwn | kOutOpp)) != (kOutOwn | kOutOpp)) {
+            const int corner = (int)(cf & kCornerMask);
             const int b = corner & 31;
             k = (b << 16) | atomicAdd(&cnt[b], 1);
             atomicAdd(&kcnt[corner], 1);
@@ -699,7 +754,17 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
 #pragma unroll
     for (int q = 0; q < kKeys; ++q) {
         const int k = key[q];
-        if (k >= 0) order[start[k >> 16] + (k & 0xffff)] = (unsigned short)(tid + q * (int)blockDim.x);
+        if (k < 0) continue;
+        const int b = k >> 16, r = k & 0xffff;  // bank, round
+        int pos = start[b] + r;
+        if constexpr (DIM == 2) {
+            // rounds one after another: points of earlier rounds, then the
+            // lower banks of this round
+            pos = 0;
+#pragma unroll
+            for (int o = 0; o < 32; ++o) pos += min(cnt[o], r) + (o < b && cnt[o] > r);
+        }
+        order[pos] = (unsigned short)(tid + q * (int)blockDim.x);
     }
     // footprints per cell: box sums of the corner histogram along each axis
     __syncthreads();
@@ -715,10 +780,11 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
     const int eb = fix_exponent_tile(mb, __int_as_float(kbin[sp.x]), eg);
     const float fscale = ldexpf(1.f, eb);
 
-    const int lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const int lane = tid & 31, warp = tid >> 5, nwarps = (int)blockDim.x >> 5;
     const unsigned sm_re = (unsigned)__cvta_generic_to_shared(are);
     const unsigned plane_bytes = 4u * (unsigned)acc_n;  // bytes between the real and imaginary planes
     const int mycnt = cnt[lane], mystart = start[lane], nrounds = maxcnt, nfull = mincnt;
+    const int npts = start[31] + cnt[31];
     // ---- rounds 0 .. nrounds-1 in passes; round r holds the banks with more
     // than r points, so the sets shrink with r.  Rounds below nfull hold every
     // bank.  In 3D the lowest tail round left (banks A_lo) takes the highest
@@ -733,7 +799,9 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
     for (int pass = warp;; pass += nwarps) {
         int i = pass, j = 0, rot = 0;
         unsigned alo = 0xffffffffu, ahi = 0;
-        if (pass >= nfull) {
+        if (DIM == 2) {
+            if (pass * 32 >= npts) break;
+        } else if (pass >= nfull) {
             bool found = false;
             while (wi <= wj) {
                 const unsigned lo = __ballot_sync(0xffffffffu, mycnt > wi);
@@ -762,7 +830,9 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
             if (!found) break;
         }
         int p = -1, prot = 0;
-        if ((alo >> lane) & 1u) {
+        if (DIM == 2) {
+            if (pass * 32 + lane < npts) p = order[pass * 32 + lane];
+        } else if ((alo >> lane) & 1u) {
             p = order[mystart + i];
         } else if (ahi) {
             const int k = __popc(~alo & ((1u << lane) - 1u));  // rank among the free lanes
@@ -772,8 +842,8 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
             }
         }
         if (p >= 0)
-            spread_point<DIM, W>(pts, g, c, cstride, nvol, perm[sp.y + p], mode, shifts, S, tx, plane, tsize,
-                                 sm_re, plane_bytes, fscale, prot);
+            spread_point<DIM, W>(pts, g, c, nvol, perm[sp.y + p], corners[sp.y + p], mode, shifts, tx, plane,
+                                 tsize, sm_re, plane_bytes, fscale, prot);
     }
     __syncthreads();
     // flush the tile's exact sums at the launch's scale (halos overlap
@@ -801,8 +871,9 @@ template <int DIM, int W>
 __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
                                                      const float2 *__restrict__ grid, long gstride,
                                                      int nvol, const int *__restrict__ perm,
-                                                     const int4 *__restrict__ subs,
-                                                     float2 *__restrict__ c, long cstride, int mode) {
+                                                     const unsigned short *__restrict__ corners,
+                                                     const int4 *__restrict__ subs, float2 *__restrict__ c,
+                                                     int mode) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *tile = reinterpret_cast<float2 *>(smem_raw);
     const int4 sp = subs[blockIdx.x];
@@ -830,8 +901,17 @@ __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
         const int j = perm[sp.y + p];
         PointInfo pi;
         point_at(pts, j, pi);
-        if (mode != PT_PLAIN && !in_band(pi)) {
-            for (int s = 0; s < nvol; ++s) c[(long)s * cstride + j] = make_float2(0.f, 0.f);
+        const unsigned out = mode == PT_PLAIN ? 0u : corners[sp.y + p];
+        // a real volume has C(-x) = conj C(x): the point's value is stored at
+        // both lattice points of the pair (zero outside the band)
+        float2 *own = c + (long)pi.angle * pts.lat + pi.l;
+        float2 *opp = c + (long)pi.angle * pts.lat + (pts.lat - 1 - pi.l);
+        const bool both = own != opp;
+        if ((out & (kOutOwn | kOutOpp)) == (kOutOwn | kOutOpp)) {
+            for (int s = 0; s < nvol; ++s) {
+                own[(long)s * pts.M] = make_float2(0.f, 0.f);
+                opp[(long)s * pts.M] = make_float2(0.f, 0.f);
+            }
             continue;
         }
         float wk[2][W];
@@ -888,20 +968,22 @@ __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
                     ai = fmaf(zi, wz, ai);
                 }
             }
-            c[(long)s * cstride + j] = make_float2(ar, ai);
+            if (pi.flip) ai = -ai;
+            own[(long)s * pts.M] = (out & kOutOwn) ? make_float2(0.f, 0.f) : make_float2(ar, ai);
+            if (both) opp[(long)s * pts.M] = (out & kOutOpp) ? make_float2(0.f, 0.f) : make_float2(ar, -ai);
         }
     }
 }
 
 template <int DIM, int W>
 void launch_spread_w(const Context &ctx, dim3 grid, size_t smem, cudaStream_t st, const PolarPts &pts,
-                     const GridCfg &g, const float2 *c, long cstride, int nvol, const int *perm,
+                     const GridCfg &g, const float2 *c, int nvol, const int *perm,
                      const unsigned short *corners, const int4 *subs, unsigned long long *out, long gstride,
                      int mode, const float2 *shifts, const int *mbits, long kmax, const int *kbin,
                      const int *binm) {
     auto kern = spread_kernel<DIM, W>;
     allow_max_dynamic_smem(ctx, kern);
-    kern<<<grid, kSpreadThreads, smem, st>>>(pts, g, c, cstride, nvol, perm, corners, subs, out, gstride,
+    kern<<<grid, kSpreadThreads, smem, st>>>(pts, g, c, nvol, perm, corners, subs, out, gstride,
                                              mode, shifts, mbits, kmax, kbin, binm);
     LC_CHECK_LAUNCH();
 }
@@ -918,10 +1000,10 @@ void launch_footprint_w(const Context &ctx, unsigned nbins, size_t smem, cudaStr
 template <int DIM, int W>
 void launch_interp_w(const Context &ctx, dim3 grid, int threads, size_t smem, cudaStream_t st,
                      const PolarPts &pts, const GridCfg &g, const float2 *gr, long gstride, int nvol,
-                     const int *perm, const int4 *subs, float2 *c, long cstride, int mode) {
+                     const int *perm, const unsigned short *corners, const int4 *subs, float2 *c, int mode) {
     auto kern = interp_kernel<DIM, W>;
     allow_max_dynamic_smem(ctx, kern);
-    kern<<<grid, threads, smem, st>>>(pts, g, gr, gstride, nvol, perm, subs, c, cstride, mode);
+    kern<<<grid, threads, smem, st>>>(pts, g, gr, gstride, nvol, perm, corners, subs, c, mode);
     LC_CHECK_LAUNCH();
 }
 
@@ -1007,7 +1089,7 @@ void NufftPlan::sort_points(Context &ctx) {
     DevBuf<int> counts(nbins, st);
     counts.zero(st);
     int threads = 256;
-    long blocks = std::min<long>((pts_.M + threads - 1) / threads, (long)ctx.num_sms() * 16);
+    long blocks = std::min<long>((pts_.Mh + threads - 1) / threads, (long)ctx.num_sms() * 16);
     blocks = std::max<long>(blocks, 1);
     if (dim_ == 2) bin_count_kernel<2><<<(unsigned)blocks, threads, 0, st>>>(pts_, g, w_, counts.get());
     else bin_count_kernel<3><<<(unsigned)blocks, threads, 0, st>>>(pts_, g, w_, counts.get());
@@ -1025,7 +1107,7 @@ void NufftPlan::sort_points(Context &ctx) {
             subs.push_back(make_int4((int)b, (int)(acc + s), std::min(maxsub, hc[b] - s), 0));
         acc += hc[b];
     }
-    LC_REQUIRE(acc == pts_.M, "NUFFT: bin sort lost points");
+    LC_REQUIRE(acc == pts_.Mh, "NUFFT: bin sort lost points");
     // footprints over one cell: a footprint reaches at most w/2 + 1 <= bs
     // cells beyond its point's cell, so only points of the bin and of its
     // neighbours (wrapped, each counted once) can cover a cell of the bin;
@@ -1051,9 +1133,9 @@ void NufftPlan::sort_points(Context &ctx) {
     subs_.upload(subs.data(), subs.size(), st);
     DevBuf<int> cursor;
     cursor.upload(off.data(), off.size(), st);
-    perm_.alloc(pts_.M, st);
-    corner_.alloc(pts_.M, st);
-    LC_REQUIRE((long)g.td[0] * g.td[1] * g.td[2] <= 65536, "NUFFT: bin tile too large for 16-bit corners");
+    perm_.alloc(pts_.Mh, st);
+    corner_.alloc(pts_.Mh, st);
+    LC_REQUIRE((long)g.td[0] * g.td[1] * g.td[2] <= (long)kCornerMask + 1, "NUFFT: bin tile too large for its corners");
     if (dim_ == 2)
         bin_scatter_kernel<2><<<(unsigned)blocks, threads, 0, st>>>(pts_, g, w_, cursor.get(), perm_.get(),
                                                                     corner_.get());
@@ -1068,7 +1150,6 @@ void NufftPlan::sort_points(Context &ctx) {
         DevBuf<int2> dbr;
         dbr.upload(br.data(), br.size(), st);
         kbin_.alloc(nbins, st);
-        binm_.alloc(nbins, st);
         LC_REQUIRE(nbins < (1L << 31), "NUFFT: too many bins");
         const size_t hsm = (size_t)g.td[0] * g.td[1] * g.td[2] * sizeof(int);
         LC_REQUIRE(hsm <= ctx.max_smem(), "NUFFT: bin tile does not fit shared memory");
@@ -1115,14 +1196,18 @@ void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, Pt
     fix_.ensure(2 * gvol * nvol, st);
     LC_CUDA(cudaMemsetAsync(mbits_.get(), 0, sizeof(int), st));
     LC_CUDA(cudaMemsetAsync(fix_.get(), 0, 2 * gvol * nvol * sizeof(long long), st));
-    {
-        const long n = (long)nvol * pts_.M;
-        const long blocks = std::max<long>(1, std::min<long>((n + 255) / 256, (long)ctx.num_sms() * 8));
-        value_bound_kernel<<<(unsigned)blocks, 256, 0, st>>>(c, n, mbits_.get());
+    const int vchunk = (int)std::max<size_t>(1, (96 * 1024) / tile_bytes);
+    const long nbins = (long)nb_[0] * nb_[1] * nb_[2];
+    // the bins' value bounds per chunk of volumes, and the launch's
+    binm_.ensure(nbins * ((nvol + vchunk - 1) / vchunk), st);
+    LC_CUDA(cudaMemsetAsync(binm_.get(), 0, binm_.size() * sizeof(int), st));
+    for (int v0 = 0; v0 < nvol; v0 += vchunk) {
+        bin_value_bound_kernel<<<nsub_, 256, 0, st>>>(pts_, c + (long)v0 * pts_.M, std::min(vchunk, nvol - v0),
+                                                      perm_.get(), corner_.get(), subs_.get(), mode,
+                                                      binm_.get() + nbins * (v0 / vchunk), mbits_.get());
         LC_CHECK_LAUNCH();
     }
     unsigned long long *fix = reinterpret_cast<unsigned long long *>(fix_.get());
-    const int vchunk = (int)std::max<size_t>(1, (96 * 1024) / tile_bytes);
     for (int v0 = 0; v0 < nvol; v0 += vchunk) {
         const int nv = std::min(vchunk, nvol - v0);
         const size_t smem = tile_bytes * nv + bucket_bytes;
@@ -1130,18 +1215,15 @@ void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, Pt
         const float2 *cv = c + (long)v0 * pts_.M;
         unsigned long long *fv = fix + 2 * (long)v0 * gvol;
         dim3 gd(nsub_);
-        // the bins' value bounds over this chunk of volumes
-        LC_CUDA(cudaMemsetAsync(binm_.get(), 0, binm_.size() * sizeof(int), st));
-        bin_value_bound_kernel<<<gd, 256, 0, st>>>(cv, pts_.M, nv, perm_.get(), subs_.get(), binm_.get());
-        LC_CHECK_LAUNCH();
+        const int *bm = binm_.get() + nbins * (v0 / vchunk);
         if (dim_ == 2) {
-            LC_W_SWITCH(w_, (launch_spread_w<2, WW>(ctx, gd, smem, st, pts_, g, cv, pts_.M, nv,
+            LC_W_SWITCH(w_, (launch_spread_w<2, WW>(ctx, gd, smem, st, pts_, g, cv, nv,
                                                    perm_.get(), corner_.get(), subs_.get(), fv, gvol, mode, shifts_,
-                                                   mbits_.get(), kmax_, kbin_.get(), binm_.get())));
+                                                   mbits_.get(), kmax_, kbin_.get(), bm)));
         } else {
-            LC_W_SWITCH(w_, (launch_spread_w<3, WW>(ctx, gd, smem, st, pts_, g, cv, pts_.M, nv,
+            LC_W_SWITCH(w_, (launch_spread_w<3, WW>(ctx, gd, smem, st, pts_, g, cv, nv,
                                                    perm_.get(), corner_.get(), subs_.get(), fv, gvol, mode, shifts_,
-                                                   mbits_.get(), kmax_, kbin_.get(), binm_.get())));
+                                                   mbits_.get(), kmax_, kbin_.get(), bm)));
         }
     }
     {
@@ -1166,10 +1248,10 @@ void NufftPlan::interp(Context &ctx, const float2 *grid, int nvol, float2 *c, Pt
         dim3 gd(nsub_);
         if (dim_ == 2) {
             LC_W_SWITCH(w_, (launch_interp_w<2, WW>(ctx, gd, 256, smem, ctx.stream(), pts_, g, gv, gvol, nv,
-                                                   perm_.get(), subs_.get(), cv, pts_.M, mode)));
+                                                   perm_.get(), corner_.get(), subs_.get(), cv, mode)));
         } else {
             LC_W_SWITCH(w_, (launch_interp_w<3, WW>(ctx, gd, 256, smem, ctx.stream(), pts_, g, gv, gvol, nv,
-                                                   perm_.get(), subs_.get(), cv, pts_.M, mode)));
+                                                   perm_.get(), corner_.get(), subs_.get(), cv, mode)));
         }
     }
 }

@@ -45,7 +45,13 @@ struct PolarPts {
     // 3D
     int nrows = 0, ncols = 0;
     const double *rot = nullptr;  // R00 R01 R10 R11 R20 R21 per angle
-    // point index -> angle (by nr in 2D, nrows * ncols in 3D) and, in 3D, row (by ncols)
+    // The lattice of an angle (lat = nr points in 2D, nrows * ncols in 3D) is
+    // closed under negation: lattice point l and lat - 1 - l are opposite.  A
+    // plan handles one point of each pair: half = ceil(lat / 2) per angle,
+    // l < half, Mh over all angles (see fold_value).
+    int lat = 0, half = 0;
+    long Mh = 0;
+    // folded point index -> angle (by half) and, in 3D, lattice point -> row (by ncols)
     FastDiv div_angle, div_col;
 };
 
@@ -107,7 +113,7 @@ class NufftPlan {
     DevBuf<float> corr_[3];
     DevBuf<float> corr_xy_;  // corr_y (x) corr_x, 3D type 2
     DevBuf<int> perm_;
-    DevBuf<unsigned short> corner_;  // per sorted point: footprint corner in its bin's tile
+    DevBuf<unsigned short> corner_;  // per sorted point: footprint corner in its bin's tile, band flags
     DevBuf<int4> subs_;
     int nsub_ = 0;
     int maxsub_ = 1024;  // most points of one spreading subproblem
@@ -116,7 +122,7 @@ class NufftPlan {
     DevBuf<long long> fix_;  // 64-bit fixed-point fine grid of the spreading (re, im)
     DevBuf<int> mbits_;      // bound on the spread values (float bits)
     DevBuf<int> kbin_;       // per bin: bound on the summed weights over one tile cell (float bits)
-    DevBuf<int> binm_;       // per bin: bound on its spread values (float bits), per call
+    DevBuf<int> binm_;       // per bin and chunk of volumes: bound on its spread values (float bits), per call
 };
 
 }  // namespace lc
