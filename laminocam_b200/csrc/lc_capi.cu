@@ -116,8 +116,11 @@ void do_backproj2d(lc_geometry g, const float *sino, int ns, int n2, int n3, flo
     d.d_pre = nr / 2;         // fftshift1
     d.d_post = (nr + 1) / 2;  // ifftshift1
     d.sign = -1;
+    // odd lines: the values at opposite radii are conjugates, so half are formed
+    const bool herm = nr % 2 == 1 && dft_on_lines(nr);
+    if (herm) d.out_max = g->g.pts.half;
     launch_axis_dft(ctx, d);
-    plan_for(g, n3, n2, 1, tol).type1_real(ctx, g->work.get(), ns, vol, 1.0f / (float)nr, PT_PLAIN);
+    plan_for(g, n3, n2, 1, tol).type1_real(ctx, g->work.get(), ns, vol, 1.0f / (float)nr, PT_PLAIN, herm);
 }
 
 void do_forward2d(lc_geometry g, const float *vol, int ns, int n2, int n3, float *sino, double tol) {
@@ -151,6 +154,9 @@ void do_backproj3d(lc_geometry g, const float *proj, int n1, int n2, int n3, boo
     const int nth = g->g.pts.ntheta, nrows = g->g.pts.nrows, ncols = g->g.pts.ncols;
     const long M = g->g.pts.M;
     g->work.ensure(M, ctx.stream());
+    // odd sides: the transform of a real image is Hermitian about the lattice's
+    // centre, so half of the columns, then half of the lattice, are formed
+    const bool herm = nrows % 2 == 1 && ncols % 2 == 1 && dft_on_lines(nrows) && dft_on_lines(ncols);
     {
         AxisDFT d;  // along ncols: fftshift -> FFT -> ifftshift
         d.in = proj;
@@ -165,6 +171,7 @@ void do_backproj3d(lc_geometry g, const float *proj, int n1, int n2, int n3, boo
         d.d_pre = ncols / 2;
         d.d_post = (ncols + 1) / 2;
         d.sign = -1;
+        if (herm) d.out_min = ncols / 2;
         launch_axis_dft(ctx, d);
     }
     {
@@ -181,11 +188,12 @@ void do_backproj3d(lc_geometry g, const float *proj, int n1, int n2, int n3, boo
         d.d_pre = nrows / 2;
         d.d_post = (nrows + 1) / 2;
         d.sign = -1;
+        d.herm = herm;
         launch_axis_dft(ctx, d);
     }
     plan_for(g, n3, n2, n1, tol).type1_real(ctx, g->work.get(), 1, vol,
                                             1.0f / ((float)nrows * (float)ncols),
-                                            shifts ? PT_SHIFT : PT_MASK);
+                                            shifts ? PT_SHIFT : PT_MASK, herm);
 }
 
 void do_forward3d(lc_geometry g, const float *vol, int n1, int n2, int n3, float *proj, double tol) {
@@ -194,14 +202,22 @@ void do_forward3d(lc_geometry g, const float *vol, int n1, int n2, int n3, float
     const int nth = g->g.pts.ntheta, nrows = g->g.pts.nrows, ncols = g->g.pts.ncols;
     const long M = g->g.pts.M;
     g->work.ensure(M, ctx.stream());
-    plan_for(g, n3, n2, n1, tol).type2_real(ctx, vol, 1, g->work.get(), PT_MASK);
+    // odd sides: the values are Hermitian about the lattice's centre, so the
+    // rows up to the centre determine the others
+    const bool herm = nrows % 2 == 1 && ncols % 2 == 1 && dft_on_lines(nrows) && dft_on_lines(ncols);
+    const int rows = herm ? nrows / 2 + 1 : nrows;
+    plan_for(g, n3, n2, n1, tol).type2_real(ctx, vol, 1, g->work.get(), PT_MASK, herm ? rows * ncols : 0);
     {
         AxisDFT d;  // along ncols: fftshift -> IFFT -> ifftshift, in place
         d.in = g->work.get();
         d.in_t = E_C64;
         d.out = g->work.get();
         d.out_t = E_C64;
-        d.n_outer = (long)nth * nrows;
+        d.n_outer = (long)nth * rows;
+        if (herm) {
+            d.rows_per = rows;
+            d.group_stride = (long)nrows * ncols;
+        }
         d.n_inner = 1;
         d.in_ostride = ncols;
         d.out_ostride = ncols;
@@ -226,6 +242,7 @@ void do_forward3d(lc_geometry g, const float *vol, int n1, int n2, int n3, float
         d.d_post = (nrows + 1) / 2;
         d.sign = +1;
         d.scale = 1.0f / ((float)nrows * (float)ncols);
+        d.herm = herm;
         launch_axis_dft(ctx, d);
     }
 }

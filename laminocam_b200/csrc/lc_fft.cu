@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "lc_fft.hpp"
+#include "lc_regfft.cuh"
 
 namespace lc {
 
@@ -992,6 +993,22 @@ __global__ void bluestein_kernel(BArgs a, FFTPlan pl) {
     }
 }
 
+// Convolution length: the next 2^p 3^q, or the next even one when that is a
+// power of three (81, 243, 729, 2187): the line kernels need an even length.
+// (Both detector passes of a 180 x 361 x 361 projection: 1.11 ms at 729 points
+// on the generic kernel, 0.33 ms at 768 on the line kernels.)
+static int bluestein_length(int n) {
+    long L = next_smooth23(2L * n - 1);
+    while (L % 2 != 0) L = next_smooth23(L + 1);
+    return (int)L;
+}
+
+bool dft_on_lines(int n) {
+    if (n < 16 || !line_kernels_enabled()) return false;
+    const int L = bluestein_length(n);
+    return L <= 8192 && n <= L / 2 && line_plan_exists(L / 2);
+}
+
 __global__ void c128_to_c64_kernel(const double2 *in, float2 *out, int n, double scale) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         out[i] = make_float2((float)(in[i].x * scale), (float)(in[i].y * scale));
@@ -1003,7 +1020,7 @@ const BluesteinEntry &bluestein_tables(Context &ctx, int n, int sign) {
     auto e = std::make_unique<BluesteinEntry>();
     e->n = n;
     e->sign = sign;
-    e->L = (int)next_smooth23(2L * n - 1);
+    e->L = bluestein_length(n);
     const int L = e->L;
     const double pi = 3.14159265358979323846;
     std::vector<double2> a(n), v(L, make_double2(0.0, 0.0));
@@ -1057,6 +1074,8 @@ void bluestein_launch(Context &ctx, const BArgs &b, const FFTPlan &pl, long bloc
 void launch_bluestein(Context &ctx, const AxisDFT &a) {
     const BluesteinEntry &e = bluestein_tables(ctx, a.n, a.sign);
     if (line_kernels_enabled() && launch_bluestein_lines(ctx.stream(), a, e)) return;
+    LC_REQUIRE(!a.herm && a.rows_per == 0 && a.out_min == 0 && a.out_max == 0,
+               "DFT: Hermitian and grouped lines need a register plan");
     const FFTPlan &pl = ctx.plans().get(e.L, false, ctx.stream());
     AxisFFT shape;  // only to pick the line grouping
     shape.L = e.L;
@@ -1105,10 +1124,12 @@ void launch_axis_dft(Context &ctx, const AxisDFT &a) {
     LC_REQUIRE(a.in_t == E_F32 || a.in_t == E_C64, "DFT input must be float or float2");
     LC_REQUIRE(a.out_t == E_F32 || a.out_t == E_C64, "DFT output must be float or float2");
     if (a.n_outer <= 0 || a.n_inner <= 0) return;
-    if (a.n >= 16 && next_smooth23(2L * a.n - 1) <= 8192) {
+    if (a.n >= 16 && bluestein_length(a.n) <= 8192) {
         launch_bluestein(ctx, a);
         return;
     }
+    LC_REQUIRE(!a.herm && a.rows_per == 0 && a.out_min == 0 && a.out_max == 0,
+               "DFT: Hermitian and grouped lines need a register plan");
     DArgs d{};
     d.in = a.in;
     d.out = a.out;

@@ -194,13 +194,30 @@ struct AxisDFT {
     int d_post = 0;  // stored line:  out[k] = DFT(v)[(k + d_post) % n]
     int sign = -1;
     float scale = 1.0f;
+    // Lines of data that is Hermitian about a stored centre; only lengths with
+    // dft_on_lines(n) take these.
+    // Rows (n_inner == 1) in groups: line g * rows_per + r is at
+    // g * group_stride + r * stride (0: the lines follow one another).
+    long rows_per = 0, group_stride = 0;
+    // Real rows: store only the outputs k in [out_min, out_max) (out_max 0: n).
+    int out_min = 0, out_max = 0;
+    // Columns of odd n_inner and odd n, out[n_inner-1-c] = conj(in[c]) reversed:
+    //   complex output: only the columns c >= n_inner / 2 are read; their
+    //     outputs at rows k <= n / 2, and the mirrored columns' outputs
+    //     out(n-1-k, n_inner-1-c) = conj out(k, c) there, are stored;
+    //   real output: only the input rows up to n / 2 are read (the input at row
+    //     n-1-k is the conjugate of that at row k).
+    bool herm = false;
 };
 
+// true when launch_axis_dft runs length n on the register-plan Bluestein
+// kernels (the Hermitian forms of AxisDFT need them)
+bool dft_on_lines(int n);
 void launch_axis_dft(Context &ctx, const AxisDFT &a);
 
-// Bluestein transforms with complex output whose convolution length is even
-// with a register plan for half of it, on the line kernels; false otherwise
-// (the generic Bluestein kernel then runs).
+// Bluestein transforms whose convolution length is even with a register plan
+// for half of it, on the line kernels; false otherwise (the generic Bluestein
+// kernel then runs).
 bool launch_bluestein_lines(cudaStream_t st, const AxisDFT &a, const BluesteinEntry &e);
 
 }  // namespace lc

@@ -209,12 +209,19 @@ constexpr unsigned kCornerMask = 0x3fffu, kOutOwn = 0x8000u, kOutOpp = 0x4000u;
 // so one point with the value c + conj(c') stands for both (its conjugate
 // when the point is negated), at half the footprints to spread: the 3D
 // spreading of 360 x 511 x 511 values onto 48 x 1024 x 1024 cells took 14.3 ms
-// with every point and 7.1 ms folded.  Values outside the band are left out; cv is the volume's value array, out the flags
-// that count.
+// with every point and 7.1 ms folded.  Values outside the band are left out;
+// cv is the volume's value array, out the flags that count.  herm: c' = conj c
+// is known and not read.
 __device__ __forceinline__ float2 fold_value(const PolarPts &p, const float2 *__restrict__ cv, int angle, int l,
-                                             unsigned out) {
+                                             unsigned out, bool herm) {
     const float2 *a = cv + (long)angle * p.lat;
     float2 v = make_float2(0.f, 0.f);
+    if (herm) {
+        const float2 w = a[l];
+        float f = (out & kOutOwn) ? 0.f : 1.f;
+        if (2 * l + 1 != p.lat && !(out & kOutOpp)) f += 1.f;
+        return make_float2(f * w.x, f * w.y);
+    }
     if (!(out & kOutOwn)) v = a[l];
     if (2 * l + 1 != p.lat && !(out & kOutOpp)) {
         const float2 w = a[p.lat - 1 - l];
@@ -507,7 +514,7 @@ __device__ __forceinline__ void rot_banks(int rot, int plane, int &d1, int &d2) 
 template <int DIM, int W>
 __device__ __forceinline__ void spread_point(const PolarPts &pts, const GridCfg &g,
                                              const float2 *__restrict__ c, int nvol, int j, unsigned cf,
-                                             int mode, const float2 *__restrict__ shifts,
+                                             int mode, bool herm, const float2 *__restrict__ shifts,
                                              int tx, int plane, int tsize, unsigned sm_re,
                                              unsigned plane_bytes, float fscale, int rot) {
     const float inv_hw = 2.0f / (float)W;
@@ -541,7 +548,7 @@ __device__ __forceinline__ void spread_point(const PolarPts &pts, const GridCfg 
         }
     }
     for (int s = 0; s < nvol; ++s) {
-        float2 v = fold_value(pts, c + (long)s * pts.M, pi.angle, pi.l, out);
+        float2 v = fold_value(pts, c + (long)s * pts.M, pi.angle, pi.l, out, herm);
         v = mode == PT_SHIFT ? cmul(v, mult) : make_float2(v.x * fscale, v.y * fscale);
         if (pi.flip) v.y = -v.y;
         // 32-bit shared addresses of the footprint corner in the two planes
@@ -649,8 +656,8 @@ __global__ void __launch_bounds__(256) bin_footprint_kernel(GridCfg g, OffsetWei
 __global__ void __launch_bounds__(256) bin_value_bound_kernel(PolarPts pts, const float2 *__restrict__ c,
                                                               int nvol, const int *__restrict__ perm,
                                                               const unsigned short *__restrict__ corners,
-                                                              const int4 *__restrict__ subs, int mode, int *binm,
-                                                              int *mbits) {
+                                                              const int4 *__restrict__ subs, int mode, int herm,
+                                                              int *binm, int *mbits) {
     __shared__ int mx;
     const int4 sp = subs[blockIdx.x];
     if (threadIdx.x == 0) mx = 0;
@@ -661,7 +668,8 @@ __global__ void __launch_bounds__(256) bin_value_bound_kernel(PolarPts pts, cons
         const unsigned i = fast_div(j, pts.div_angle);
         const unsigned out = mode == PT_PLAIN ? 0u : corners[sp.y + p];
         for (int s = 0; s < nvol; ++s) {
-            const float2 v = fold_value(pts, c + (long)s * pts.M, (int)i, (int)(j - i * (unsigned)pts.half), out);
+            const float2 v = fold_value(pts, c + (long)s * pts.M, (int)i, (int)(j - i * (unsigned)pts.half), out,
+                                        herm != 0);
             m = fmaxf(m, fabsf(v.x) + fabsf(v.y));
         }
     }
@@ -684,7 +692,7 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
     spread_kernel(PolarPts pts, GridCfg g, const float2 *__restrict__ c, int nvol,
                   const int *__restrict__ perm, const unsigned short *__restrict__ corners,
                   const int4 *__restrict__ subs,
-                  unsigned long long *__restrict__ fix, long gstride, int mode,
+                  unsigned long long *__restrict__ fix, long gstride, int mode, int herm,
                   const float2 *__restrict__ shifts, const int *__restrict__ mbits, long kmax,
                   const int *__restrict__ kbin, const int *__restrict__ binm) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -842,8 +850,8 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
             }
         }
         if (p >= 0)
-            spread_point<DIM, W>(pts, g, c, nvol, perm[sp.y + p], corners[sp.y + p], mode, shifts, tx, plane,
-                                 tsize, sm_re, plane_bytes, fscale, prot);
+            spread_point<DIM, W>(pts, g, c, nvol, perm[sp.y + p], corners[sp.y + p], mode, herm != 0, shifts,
+                                 tx, plane, tsize, sm_re, plane_bytes, fscale, prot);
     }
     __syncthreads();
     // flush the tile's exact sums at the launch's scale (halos overlap
@@ -873,7 +881,7 @@ __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
                                                      int nvol, const int *__restrict__ perm,
                                                      const unsigned short *__restrict__ corners,
                                                      const int4 *__restrict__ subs, float2 *__restrict__ c,
-                                                     int mode) {
+                                                     int mode, int keep) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *tile = reinterpret_cast<float2 *>(smem_raw);
     const int4 sp = subs[blockIdx.x];
@@ -906,11 +914,11 @@ __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
         // both lattice points of the pair (zero outside the band)
         float2 *own = c + (long)pi.angle * pts.lat + pi.l;
         float2 *opp = c + (long)pi.angle * pts.lat + (pts.lat - 1 - pi.l);
-        const bool both = own != opp;
+        const bool both = own != opp && pts.lat - 1 - pi.l < keep;
         if ((out & (kOutOwn | kOutOpp)) == (kOutOwn | kOutOpp)) {
             for (int s = 0; s < nvol; ++s) {
                 own[(long)s * pts.M] = make_float2(0.f, 0.f);
-                opp[(long)s * pts.M] = make_float2(0.f, 0.f);
+                if (both) opp[(long)s * pts.M] = make_float2(0.f, 0.f);
             }
             continue;
         }
@@ -979,12 +987,12 @@ template <int DIM, int W>
 void launch_spread_w(const Context &ctx, dim3 grid, size_t smem, cudaStream_t st, const PolarPts &pts,
                      const GridCfg &g, const float2 *c, int nvol, const int *perm,
                      const unsigned short *corners, const int4 *subs, unsigned long long *out, long gstride,
-                     int mode, const float2 *shifts, const int *mbits, long kmax, const int *kbin,
+                     int mode, int herm, const float2 *shifts, const int *mbits, long kmax, const int *kbin,
                      const int *binm) {
     auto kern = spread_kernel<DIM, W>;
     allow_max_dynamic_smem(ctx, kern);
     kern<<<grid, kSpreadThreads, smem, st>>>(pts, g, c, nvol, perm, corners, subs, out, gstride,
-                                             mode, shifts, mbits, kmax, kbin, binm);
+                                             mode, herm, shifts, mbits, kmax, kbin, binm);
     LC_CHECK_LAUNCH();
 }
 
@@ -1000,10 +1008,10 @@ void launch_footprint_w(const Context &ctx, unsigned nbins, size_t smem, cudaStr
 template <int DIM, int W>
 void launch_interp_w(const Context &ctx, dim3 grid, int threads, size_t smem, cudaStream_t st,
                      const PolarPts &pts, const GridCfg &g, const float2 *gr, long gstride, int nvol,
-                     const int *perm, const unsigned short *corners, const int4 *subs, float2 *c, int mode) {
+                     const int *perm, const unsigned short *corners, const int4 *subs, float2 *c, int mode, int keep) {
     auto kern = interp_kernel<DIM, W>;
     allow_max_dynamic_smem(ctx, kern);
-    kern<<<grid, threads, smem, st>>>(pts, g, gr, gstride, nvol, perm, corners, subs, c, mode);
+    kern<<<grid, threads, smem, st>>>(pts, g, gr, gstride, nvol, perm, corners, subs, c, mode, keep);
     LC_CHECK_LAUNCH();
 }
 
@@ -1177,7 +1185,7 @@ void NufftPlan::sort_points(Context &ctx) {
     }
 }
 
-void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, PtMode mode) {
+void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, PtMode mode, bool herm) {
     GridCfg g = make_cfg(dim_, nf_, bs_, nb_, w_, beta_);
     const long gvol = (long)nf_[0] * nf_[1] * nf_[2];
     cudaStream_t st = ctx.stream();
@@ -1203,7 +1211,7 @@ void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, Pt
     LC_CUDA(cudaMemsetAsync(binm_.get(), 0, binm_.size() * sizeof(int), st));
     for (int v0 = 0; v0 < nvol; v0 += vchunk) {
         bin_value_bound_kernel<<<nsub_, 256, 0, st>>>(pts_, c + (long)v0 * pts_.M, std::min(vchunk, nvol - v0),
-                                                      perm_.get(), corner_.get(), subs_.get(), mode,
+                                                      perm_.get(), corner_.get(), subs_.get(), mode, herm ? 1 : 0,
                                                       binm_.get() + nbins * (v0 / vchunk), mbits_.get());
         LC_CHECK_LAUNCH();
     }
@@ -1218,11 +1226,11 @@ void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, Pt
         const int *bm = binm_.get() + nbins * (v0 / vchunk);
         if (dim_ == 2) {
             LC_W_SWITCH(w_, (launch_spread_w<2, WW>(ctx, gd, smem, st, pts_, g, cv, nv,
-                                                   perm_.get(), corner_.get(), subs_.get(), fv, gvol, mode, shifts_,
+                                                   perm_.get(), corner_.get(), subs_.get(), fv, gvol, mode, herm ? 1 : 0, shifts_,
                                                    mbits_.get(), kmax_, kbin_.get(), bm)));
         } else {
             LC_W_SWITCH(w_, (launch_spread_w<3, WW>(ctx, gd, smem, st, pts_, g, cv, nv,
-                                                   perm_.get(), corner_.get(), subs_.get(), fv, gvol, mode, shifts_,
+                                                   perm_.get(), corner_.get(), subs_.get(), fv, gvol, mode, herm ? 1 : 0, shifts_,
                                                    mbits_.get(), kmax_, kbin_.get(), bm)));
         }
     }
@@ -1234,7 +1242,7 @@ void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, Pt
     }
 }
 
-void NufftPlan::interp(Context &ctx, const float2 *grid, int nvol, float2 *c, PtMode mode) {
+void NufftPlan::interp(Context &ctx, const float2 *grid, int nvol, float2 *c, PtMode mode, int keep) {
     GridCfg g = make_cfg(dim_, nf_, bs_, nb_, w_, beta_);
     const long gvol = (long)nf_[0] * nf_[1] * nf_[2];
     ProfScope ps(ctx, PS_INTERP, (double)nvol * (8.0 * pts_.M + 8.0 * gvol) + 4.0 * pts_.M);
@@ -1248,20 +1256,20 @@ void NufftPlan::interp(Context &ctx, const float2 *grid, int nvol, float2 *c, Pt
         dim3 gd(nsub_);
         if (dim_ == 2) {
             LC_W_SWITCH(w_, (launch_interp_w<2, WW>(ctx, gd, 256, smem, ctx.stream(), pts_, g, gv, gvol, nv,
-                                                   perm_.get(), corner_.get(), subs_.get(), cv, mode)));
+                                                   perm_.get(), corner_.get(), subs_.get(), cv, mode, keep)));
         } else {
             LC_W_SWITCH(w_, (launch_interp_w<3, WW>(ctx, gd, 256, smem, ctx.stream(), pts_, g, gv, gvol, nv,
-                                                   perm_.get(), corner_.get(), subs_.get(), cv, mode)));
+                                                   perm_.get(), corner_.get(), subs_.get(), cv, mode, keep)));
         }
     }
 }
 
 void NufftPlan::type1_real(Context &ctx, const float2 *c, int nvol, float *out, float scale,
-                           PtMode mode) {
+                           PtMode mode, bool herm) {
     cudaStream_t st = ctx.stream();
     const long gvol = (long)nf_[0] * nf_[1] * nf_[2];
     grid_.ensure(gvol * nvol, st);
-    spread(ctx, c, nvol, grid_.get(), mode);
+    spread(ctx, c, nvol, grid_.get(), mode, herm);
     const int n3 = modes_[0], n2 = modes_[1], n1 = modes_[2];
     const int fx = nf_[0], fy = nf_[1], fz = nf_[2];
     ProfScope ps(ctx, PS_NUFFT_FFT,
@@ -1347,7 +1355,9 @@ void NufftPlan::type1_real(Context &ctx, const float2 *c, int nvol, float *out, 
     }
 }
 
-void NufftPlan::type2_real(Context &ctx, const float *in, int nvol, float2 *c, PtMode mode) {
+void NufftPlan::type2_real(Context &ctx, const float *in, int nvol, float2 *c, PtMode mode, int keep) {
+    LC_REQUIRE(keep == 0 || (keep >= pts_.half && keep <= pts_.lat), "NUFFT: bad count of kept lattice points");
+    if (keep == 0) keep = pts_.lat;
     cudaStream_t st = ctx.stream();
     const int n3 = modes_[0], n2 = modes_[1], n1 = modes_[2];
     const int fx = nf_[0], fy = nf_[1], fz = nf_[2];
@@ -1433,7 +1443,7 @@ void NufftPlan::type2_real(Context &ctx, const float *in, int nvol, float2 *c, P
         launch_axis_fft(ctx, a);
     }
     ps.reset();
-    interp(ctx, grid_.get(), nvol, c, mode);
+    interp(ctx, grid_.get(), nvol, c, mode, keep);
 }
 
 }  // namespace lc

@@ -85,11 +85,14 @@ enum PtMode {
 class NufftPlan {
   public:
     NufftPlan(Context &ctx, const PolarGeometry &g, const int modes[3], double tol);
-    // type 1: c [nvol][M] complex -> out real [nvol][n1][n2][n3] = Re(f) * scale
+    // type 1: c [nvol][M] complex -> out real [nvol][n1][n2][n3] = Re(f) * scale.
+    // herm: the values at opposite lattice points are conjugates; only lattice
+    // points below half are read.
     void type1_real(Context &ctx, const float2 *c, int nvol, float *out, float scale,
-                    PtMode mode);
-    // type 2: real in [nvol][...modes] -> c [nvol][M]
-    void type2_real(Context &ctx, const float *in, int nvol, float2 *c, PtMode mode);
+                    PtMode mode, bool herm = false);
+    // type 2: real in [nvol][...modes] -> c [nvol][M].  keep > 0: only lattice
+    // points below it (and at least half) are stored.
+    void type2_real(Context &ctx, const float *in, int nvol, float2 *c, PtMode mode, int keep = 0);
 
     int dim() const { return dim_; }
     long M() const { return pts_.M; }
@@ -98,8 +101,8 @@ class NufftPlan {
 
   private:
     void sort_points(Context &ctx);
-    void spread(Context &ctx, const float2 *c, int nvol, float2 *grid, PtMode mode);
-    void interp(Context &ctx, const float2 *grid, int nvol, float2 *c, PtMode mode);
+    void spread(Context &ctx, const float2 *c, int nvol, float2 *grid, PtMode mode, bool herm);
+    void interp(Context &ctx, const float2 *grid, int nvol, float2 *c, PtMode mode, int keep);
 
     int dim_;
     PolarPts pts_;
