@@ -44,7 +44,7 @@ struct KArgs {
     void *out;
     long n_outer, n_inner, in_ostride, out_ostride;
     int n_in, n_out, L;
-    int in_map, out_map, out_off, sign, sign2;
+    int in_map, out_map, out_off, in_shift, out_shift, sign, sign2;
     const void *pre, *linefac, *post;
     double scale;
     const float *mid;
@@ -98,8 +98,8 @@ __device__ __forceinline__ void axis_fft_body(const KArgs &a, const FFTPlan &pl,
         gap0 = a.n_in;
         gap1 = L;
     } else if (a.in_map == IN_MODES) {
-        gap0 = a.n_in - a.n_in / 2;
-        gap1 = L - a.n_in / 2;
+        gap0 = a.n_in - a.in_shift;
+        gap1 = L - a.in_shift;
     } else if (a.in_map == IN_REAL_PACKED) {
         gap0 = (a.n_in + 1) / 2;
         gap1 = L;
@@ -162,7 +162,7 @@ __device__ __forceinline__ void axis_fft_body(const KArgs &a, const FFTPlan &pl,
                     else if (linefac) v[u] = cscale(v[u], lf);
                     int f = e;
                     if (a.in_map == IN_MODES) {
-                        f = e - a.n_in / 2;
+                        f = e - a.in_shift;
                         if (f < 0) f += L;
                     }
                     dst[u] = (f << logC) + cl;
@@ -201,7 +201,7 @@ __device__ __forceinline__ void axis_fft_body(const KArgs &a, const FFTPlan &pl,
                     }
                     int f = e;
                     if (a.in_map == IN_MODES) {
-                        f = e - a.n_in / 2;
+                        f = e - a.in_shift;
                         if (f < 0) f += L;
                     }
                     dst[u] = (f << logC) + cl;
@@ -236,7 +236,7 @@ __device__ __forceinline__ void axis_fft_body(const KArgs &a, const FFTPlan &pl,
     auto fidx = [&](int j) {
         int f = j;
         if (a.out_map == OUT_MODES) {
-            f = j - a.n_out / 2;
+            f = j - a.out_shift;
             if (f < 0) f += L;
         } else if (a.out_map == OUT_WINDOW) {
             f = j + a.out_off;
@@ -364,6 +364,8 @@ KArgs make_kargs(const AxisFFT &a, int logC, long &blocks) {
     ka.in_map = a.in_map;
     ka.out_map = a.out_map;
     ka.out_off = a.out_off;
+    ka.in_shift = a.in_shift >= 0 ? a.in_shift : a.n_in / 2;
+    ka.out_shift = a.out_shift >= 0 ? a.out_shift : a.n_out / 2;
     ka.sign = a.sign;
     ka.sign2 = a.sign2;
     ka.pre = a.pre;
@@ -756,6 +758,8 @@ void launch_axis_fft_f32_with_plan(cudaStream_t stream, size_t max_smem, const A
     ka.in_map = a.in_map;
     ka.out_map = a.out_map;
     ka.out_off = a.out_off;
+    ka.in_shift = a.in_shift >= 0 ? a.in_shift : a.n_in / 2;
+    ka.out_shift = a.out_shift >= 0 ? a.out_shift : a.n_out / 2;
     ka.sign = a.sign;
     ka.sign2 = a.sign2;
     ka.pre = a.pre;

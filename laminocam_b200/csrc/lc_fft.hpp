@@ -25,11 +25,13 @@ enum OutMap { OUT_DIRECT = 0, OUT_MODES = 1, OUT_WINDOW = 2, OUT_R2C_UNPACK = 3,
 //
 // Input maps (element j of the input line -> FFT index f):
 //   IN_DIRECT  f = j (j < n_in, zero padded to L)
-//   IN_MODES   f = (j - n_in/2) mod L        (mode k = j - floor(n_in/2))
+//   IN_MODES   f = (j - in_shift) mod L      (in_shift < 0: n_in/2, so that j is
+//              mode k = j - floor(n_in/2))
 //   IN_HERM    f in [0, L): in[f] for f <= L/2, conj(in[L-f]) otherwise
 //              (n_in = L/2 + 1, half spectrum of a real line)
 // Output maps (output element j <- FFT index f):
-//   OUT_DIRECT f = j; OUT_MODES f = (j - n_out/2) mod L; OUT_WINDOW f = j + out_off
+//   OUT_DIRECT f = j; OUT_MODES f = (j - out_shift) mod L (out_shift < 0: n_out/2);
+//   OUT_WINDOW f = j + out_off
 //
 // Real lines of even length N = 2L as complex transforms of length L (rows
 // only; the usual even/odd packing):
@@ -52,6 +54,7 @@ struct AxisFFT {
     InMap in_map = IN_DIRECT;
     OutMap out_map = OUT_DIRECT;
     int out_off = 0;
+    int in_shift = -1, out_shift = -1;
     int sign = -1;
     const void *pre = nullptr;      // real factor per input index j
     const void *linefac = nullptr;  // real factor per line inner index c

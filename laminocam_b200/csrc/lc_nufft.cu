@@ -139,6 +139,7 @@ struct GridCfg {
     int nb[3];
     int hw[3];
     int td[3];   // tile extent per dim
+    int ylo, ny;  // rows kept of the fine grid: ny from row -ylo (mod nf[1])
     double inv_nf[3];
     FastDiv div_tx, div_ty;  // by the tile extents along x and y
     float beta_l2e;          // ES beta times log2(e)
@@ -256,15 +257,19 @@ __device__ __forceinline__ int wrap_near(int v, int n) {
     return v;
 }
 
-// fine-grid offset of tile cell rr (x fastest) of the tile starting at S
+// offset in the kept part of the fine grid of tile cell rr (x fastest) of the
+// tile starting at S; negative for a cell of a row that is not kept (no
+// footprint covers it)
 template <int DIM>
 __device__ __forceinline__ long tile_cell_to_grid(int rr, const GridCfg &g, const int (&S)[3]) {
     const unsigned q = fast_div((unsigned)rr, g.div_tx);  // row of the tile: iy + ty iz
     const int ix = rr - (int)q * g.td[0];
     const unsigned iz = DIM == 3 ? fast_div(q, g.div_ty) : 0u;
     const int iy = (int)q - (int)iz * g.td[1];
-    long gi = (long)wrap_near(S[0] + ix, g.nf[0]) + (long)wrap_near(S[1] + iy, g.nf[1]) * g.nf[0];
-    if (DIM == 3) gi += (long)wrap_near(S[2] + (int)iz, g.nf[2]) * ((long)g.nf[0] * g.nf[1]);
+    const int row = wrap_near(S[1] + iy + g.ylo, g.nf[1]);
+    if (row >= g.ny) return -1;
+    long gi = (long)wrap_near(S[0] + ix, g.nf[0]) + (long)row * g.nf[0];
+    if (DIM == 3) gi += (long)wrap_near(S[2] + (int)iz, g.nf[2]) * ((long)g.nf[0] * g.ny);
     return gi;
 }
 
@@ -866,7 +871,9 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
             const int idx = s * tsize + rr;
             const int t1 = (int)((unsigned)are[idx] - kb), t2 = (int)((unsigned)aim[idx] - kb);
             if ((t1 | t2) == 0) continue;
-            unsigned long long *cell = fix + 2 * ((long)s * gstride + tile_cell_to_grid<DIM>(rr, g, S));
+            const long gi = tile_cell_to_grid<DIM>(rr, g, S);
+            if (gi < 0) continue;
+            unsigned long long *cell = fix + 2 * ((long)s * gstride + gi);
             // two's-complement sums: shift the 64-bit patterns (sh <= 40)
             if (t1) atomicAdd(cell, (unsigned long long)(long long)t1 << sh);
             if (t2) atomicAdd(cell + 1, (unsigned long long)(long long)t2 << sh);
@@ -901,8 +908,10 @@ __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
     const int tx = g.td[0], ty = g.td[1], tz = DIM == 3 ? g.td[2] : 1;
     const int tsize = tx * ty * tz;
     for (int s = 0; s < nvol; ++s)
-        for (int r = threadIdx.x; r < tsize; r += blockDim.x)
-            tile[s * tsize + r] = __ldg(grid + (long)s * gstride + tile_cell_to_grid<DIM>(r, g, S));
+        for (int r = threadIdx.x; r < tsize; r += blockDim.x) {
+            const long gi = tile_cell_to_grid<DIM>(r, g, S);
+            tile[s * tsize + r] = gi < 0 ? make_float2(0.f, 0.f) : __ldg(grid + (long)s * gstride + gi);
+        }
     __syncthreads();
     const float inv_hw = 2.0f / (float)W;
     for (int p = threadIdx.x; p < sp.z; p += blockDim.x) {
@@ -1029,8 +1038,10 @@ void launch_interp_w(const Context &ctx, dim3 grid, int threads, size_t smem, cu
         default: throw Error(1, "unsupported ES kernel width"); \
     }
 
-GridCfg make_cfg(int dim, const int nf[3], const int bs[3], const int nb[3], int w, double beta) {
+GridCfg make_cfg(int dim, const int nf[3], const int bs[3], const int nb[3], int w, double beta, int ylo, int ny) {
     GridCfg g{};
+    g.ylo = ylo;
+    g.ny = ny;
     // A point in cell c covers cells [c - floor(w/2), c + ceil(w/2)] (first
     // covered cell ceil(u - w/2) for u in [c, c+1)), so a bin of bs cells
     // needs a tile of bs + w cells starting floor(w/2) cells before it.
@@ -1065,6 +1076,17 @@ NufftPlan::NufftPlan(Context &ctx, const PolarGeometry &g, const int modes[3], d
         LC_REQUIRE(modes_[d] >= 1, "NUFFT: mode counts must be positive");
         nf_[d] = d < dim_ ? (int)next_smooth23(std::max(2 * modes_[d], 2 * w_)) : 1;
     }
+    // Folded points have u = y nf / 2 pi in [0, nf / 2] up to rounding, so
+    // footprints cover the rows -w/2 - 1 .. nf/2 + w/2 + 2 at most.  Only those
+    // are stored, cleared, converted and transformed along x; the y pass takes
+    // (type 1) or leaves (type 2) them as a window.  (Backprojection of four
+    // 1023^2 slices, 4 x 2048^2 cells: 0.59 -> 0.44 ms.)
+    ylo_ = w_ / 2 + 1;
+    ny_ = nf_[1] / 2 + 2 * (w_ / 2) + 4;
+    if (ny_ >= nf_[1]) {
+        ylo_ = 0;
+        ny_ = nf_[1];
+    }
     const int bs2[3] = {32, 32, 1};
     const int bs3[3] = {16, 8, 8};
     maxsub_ = dim_ == 2 ? 1024 : 2048;
@@ -1093,7 +1115,7 @@ NufftPlan::NufftPlan(Context &ctx, const PolarGeometry &g, const int modes[3], d
 void NufftPlan::sort_points(Context &ctx) {
     cudaStream_t st = ctx.stream();
     long nbins = (long)nb_[0] * nb_[1] * nb_[2];
-    GridCfg g = make_cfg(dim_, nf_, bs_, nb_, w_, beta_);
+    GridCfg g = make_cfg(dim_, nf_, bs_, nb_, w_, beta_, ylo_, ny_);
     DevBuf<int> counts(nbins, st);
     counts.zero(st);
     int threads = 256;
@@ -1186,8 +1208,8 @@ void NufftPlan::sort_points(Context &ctx) {
 }
 
 void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, PtMode mode, bool herm) {
-    GridCfg g = make_cfg(dim_, nf_, bs_, nb_, w_, beta_);
-    const long gvol = (long)nf_[0] * nf_[1] * nf_[2];
+    GridCfg g = make_cfg(dim_, nf_, bs_, nb_, w_, beta_, ylo_, ny_);
+    const long gvol = (long)nf_[0] * ny_ * nf_[2];
     cudaStream_t st = ctx.stream();
     // values read once, fine grid written once (plus the permutation)
     ProfScope ps(ctx, PS_SPREAD, (double)nvol * (8.0 * pts_.M + 8.0 * gvol) + 4.0 * pts_.M);
@@ -1243,8 +1265,8 @@ void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, Pt
 }
 
 void NufftPlan::interp(Context &ctx, const float2 *grid, int nvol, float2 *c, PtMode mode, int keep) {
-    GridCfg g = make_cfg(dim_, nf_, bs_, nb_, w_, beta_);
-    const long gvol = (long)nf_[0] * nf_[1] * nf_[2];
+    GridCfg g = make_cfg(dim_, nf_, bs_, nb_, w_, beta_, ylo_, ny_);
+    const long gvol = (long)nf_[0] * ny_ * nf_[2];
     ProfScope ps(ctx, PS_INTERP, (double)nvol * (8.0 * pts_.M + 8.0 * gvol) + 4.0 * pts_.M);
     const size_t tile_bytes = (size_t)g.td[0] * g.td[1] * g.td[2] * sizeof(float2);
     int vchunk = (int)std::max<size_t>(1, (96 * 1024) / tile_bytes);
@@ -1267,23 +1289,23 @@ void NufftPlan::interp(Context &ctx, const float2 *grid, int nvol, float2 *c, Pt
 void NufftPlan::type1_real(Context &ctx, const float2 *c, int nvol, float *out, float scale,
                            PtMode mode, bool herm) {
     cudaStream_t st = ctx.stream();
-    const long gvol = (long)nf_[0] * nf_[1] * nf_[2];
+    const long gvol = (long)nf_[0] * ny_ * nf_[2];
     grid_.ensure(gvol * nvol, st);
     spread(ctx, c, nvol, grid_.get(), mode, herm);
     const int n3 = modes_[0], n2 = modes_[1], n1 = modes_[2];
-    const int fx = nf_[0], fy = nf_[1], fz = nf_[2];
+    const int fx = nf_[0], fy = nf_[1], fz = nf_[2], ny = ny_;
     ProfScope ps(ctx, PS_NUFFT_FFT,
-                 (double)nvol * 8.0 * ((double)gvol + 2.0 * fz * fy * n3 + 2.0 * fz * n2 * n3) +
+                 (double)nvol * 8.0 * ((double)gvol + 2.0 * fz * ny * n3 + 2.0 * fz * n2 * n3) +
                      (double)nvol * 4.0 * n1 * n2 * n3);
     // x pass: fine rows -> n3 modes
-    h1_.ensure((long)nvol * fz * fy * n3, st);
+    h1_.ensure((long)nvol * fz * ny * n3, st);
     {
         AxisFFT a;
         a.in = grid_.get();
         a.in_t = E_C64;
         a.out = h1_.get();
         a.out_t = E_C64;
-        a.n_outer = (long)nvol * fz * fy;
+        a.n_outer = (long)nvol * fz * ny;
         a.n_inner = 1;
         a.in_ostride = fx;
         a.out_ostride = n3;
@@ -1303,9 +1325,11 @@ void NufftPlan::type1_real(Context &ctx, const float2 *c, int nvol, float *out, 
         a.out_t = E_F32;
         a.n_outer = nvol;
         a.n_inner = n3;
-        a.in_ostride = (long)fy * n3;
+        a.in_ostride = (long)ny * n3;
         a.out_ostride = (long)n2 * n3;
-        a.n_in = fy;
+        a.n_in = ny;
+        a.in_map = IN_MODES;
+        a.in_shift = ylo_;
         a.L = fy;
         a.n_out = n2;
         a.out_map = OUT_MODES;
@@ -1324,9 +1348,11 @@ void NufftPlan::type1_real(Context &ctx, const float2 *c, int nvol, float *out, 
         a.out_t = E_C64;
         a.n_outer = (long)nvol * fz;
         a.n_inner = n3;
-        a.in_ostride = (long)fy * n3;
+        a.in_ostride = (long)ny * n3;
         a.out_ostride = (long)n2 * n3;
-        a.n_in = fy;
+        a.n_in = ny;
+        a.in_map = IN_MODES;
+        a.in_shift = ylo_;
         a.L = fy;
         a.n_out = n2;
         a.out_map = OUT_MODES;
@@ -1360,13 +1386,13 @@ void NufftPlan::type2_real(Context &ctx, const float *in, int nvol, float2 *c, P
     if (keep == 0) keep = pts_.lat;
     cudaStream_t st = ctx.stream();
     const int n3 = modes_[0], n2 = modes_[1], n1 = modes_[2];
-    const int fx = nf_[0], fy = nf_[1], fz = nf_[2];
-    const long gvol = (long)fx * fy * fz;
+    const int fx = nf_[0], fy = nf_[1], fz = nf_[2], ny = ny_;
+    const long gvol = (long)fx * ny * fz;
     grid_.ensure(gvol * nvol, st);
-    h1_.ensure((long)nvol * fz * fy * n3, st);
+    h1_.ensure((long)nvol * fz * ny * n3, st);
     std::unique_ptr<ProfScope> ps(new ProfScope(
         ctx, PS_NUFFT_FFT,
-        (double)nvol * 8.0 * ((double)gvol + 2.0 * fz * fy * n3 + 2.0 * fz * n2 * n3) +
+        (double)nvol * 8.0 * ((double)gvol + 2.0 * fz * ny * n3 + 2.0 * fz * n2 * n3) +
             (double)nvol * 4.0 * n1 * n2 * n3));
     if (dim_ == 2) {
         AxisFFT a;
@@ -1377,11 +1403,13 @@ void NufftPlan::type2_real(Context &ctx, const float *in, int nvol, float2 *c, P
         a.n_outer = nvol;
         a.n_inner = n3;
         a.in_ostride = (long)n2 * n3;
-        a.out_ostride = (long)fy * n3;
+        a.out_ostride = (long)ny * n3;
         a.n_in = n2;
         a.in_map = IN_MODES;
         a.L = fy;
-        a.n_out = fy;
+        a.n_out = ny;
+        a.out_map = OUT_MODES;
+        a.out_shift = ylo_;
         a.sign = -1;
         a.pre = corr_[1].get();
         a.linefac = corr_[0].get();
@@ -1416,11 +1444,13 @@ void NufftPlan::type2_real(Context &ctx, const float *in, int nvol, float2 *c, P
             a.n_outer = (long)nvol * fz;
             a.n_inner = n3;
             a.in_ostride = (long)n2 * n3;
-            a.out_ostride = (long)fy * n3;
+            a.out_ostride = (long)ny * n3;
             a.n_in = n2;
             a.in_map = IN_MODES;
             a.L = fy;
-            a.n_out = fy;
+            a.n_out = ny;
+            a.out_map = OUT_MODES;
+            a.out_shift = ylo_;
             a.sign = -1;
             launch_axis_fft(ctx, a);
         }
@@ -1431,7 +1461,7 @@ void NufftPlan::type2_real(Context &ctx, const float *in, int nvol, float2 *c, P
         a.in_t = E_C64;
         a.out = grid_.get();
         a.out_t = E_C64;
-        a.n_outer = (long)nvol * fz * fy;
+        a.n_outer = (long)nvol * fz * ny;
         a.n_inner = 1;
         a.in_ostride = n3;
         a.out_ostride = fx;

@@ -111,6 +111,7 @@ class NufftPlan {
     int nf_[3];
     int w_;
     double beta_;
+    int ny_, ylo_;  // fine-grid rows kept: ny_ rows from row -ylo_ (mod nf_[1])
     int bs_[3];
     int nb_[3];
     DevBuf<float> corr_[3];
