@@ -471,6 +471,38 @@ __device__ __forceinline__ void spread_row(unsigned re, unsigned im, float vr, f
     }
 }
 
+// Order of a CTA's points by shared-memory bank: point rank r of bank b
+// (corner index mod 32) goes to position S(r) + (banks below b that hold more
+// than r points), S(r) the points of rank below r, so that consecutive lanes
+// hold distinct banks while every bank lasts.  fill() tabulates the first
+// ranks; both read cnt, the points per bank.
+constexpr int kBankTab = 256;
+struct BankTable {
+    int before[kBankTab];
+    unsigned banks[kBankTab];
+};
+
+__device__ __forceinline__ void bank_table_fill(BankTable &t, const int *cnt, int ranks) {
+    for (int r = threadIdx.x; r < min(ranks, kBankTab); r += blockDim.x) {
+        int s = 0;
+        unsigned m = 0;
+#pragma unroll
+        for (int o = 0; o < 32; ++o) {
+            s += min(cnt[o], r);
+            m |= (cnt[o] > r ? 1u : 0u) << o;
+        }
+        t.before[r] = s;
+        t.banks[r] = m;
+    }
+}
+
+__device__ __forceinline__ int bank_position(const BankTable &t, const int *cnt, int b, int r) {
+    if (r < kBankTab) return t.before[r] + __popc(t.banks[r] & ((1u << b) - 1u));
+    int pos = 0;
+    for (int o = 0; o < 32; ++o) pos += min(cnt[o], r) + (o < b && cnt[o] > r ? 1 : 0);
+    return pos;
+}
+
 // cnt[q] <- sum of cnt[q - d], d in [0, w), along one axis of a tile of
 // tx x ty x tz cells (in place: a thread walks each of its lines downwards
 // with a sliding window, so the values it still reads are the original ones)
@@ -702,6 +734,7 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
                   const int *__restrict__ kbin, const int *__restrict__ binm) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int cnt[32], start[32], mincnt, maxcnt;
+    __shared__ BankTable btab;  // 2D
     const int4 sp = subs[blockIdx.x];
     int bcoord[3] = {0, 0, 0};
     {
@@ -764,20 +797,16 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
         }
     }
     __syncthreads();
+    if constexpr (DIM == 2) {
+        bank_table_fill(btab, cnt, maxcnt);
+        __syncthreads();
+    }
 #pragma unroll
     for (int q = 0; q < kKeys; ++q) {
         const int k = key[q];
         if (k < 0) continue;
         const int b = k >> 16, r = k & 0xffff;  // bank, round
-        int pos = start[b] + r;
-        if constexpr (DIM == 2) {
-            // rounds one after another: points of earlier rounds, then the
-            // lower banks of this round
-            pos = 0;
-#pragma unroll
-            for (int o = 0; o < 32; ++o) pos += min(cnt[o], r) + (o < b && cnt[o] > r);
-        }
-        order[pos] = (unsigned short)(tid + q * (int)blockDim.x);
+        order[DIM == 2 ? bank_position(btab, cnt, b, r) : start[b] + r] = (unsigned short)(tid + q * (int)blockDim.x);
     }
     // footprints per cell: box sums of the corner histogram along each axis
     __syncthreads();
@@ -882,6 +911,12 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
 }
 
 // ---- interpolation --------------------------------------------------------
+// One thread gathers one point's footprint from the bin's tile in shared
+// memory.  The gathers bound the kernel: with the points in bin order they ran
+// at 96 % of the shared-memory wavefronts, 59 % of them replays of bank
+// conflicts, so the points are taken in bank order (BankTable): a half warp's
+// 8-byte loads then fall in distinct bank pairs.  (Projection 180 x 361 x 361:
+// 2.75 -> 2.11 ms; four 511^2 slices: 0.108 -> 0.099 ms.)
 template <int DIM, int W>
 __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
                                                      const float2 *__restrict__ grid, long gstride,
@@ -890,6 +925,8 @@ __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
                                                      const int4 *__restrict__ subs, float2 *__restrict__ c,
                                                      int mode, int keep) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int cnt[32];
+    __shared__ BankTable btab;
     float2 *tile = reinterpret_cast<float2 *>(smem_raw);
     const int4 sp = subs[blockIdx.x];
     const int bin = sp.x;
@@ -907,14 +944,35 @@ __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
     for (int d = 0; d < DIM; ++d) S[d] = bcoord[d] * g.bs[d] - g.hw[d];
     const int tx = g.td[0], ty = g.td[1], tz = DIM == 3 ? g.td[2] : 1;
     const int tsize = tx * ty * tz;
+    unsigned short *order = reinterpret_cast<unsigned short *>(tile + (long)nvol * tsize);
+    if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    int key[8];  // (bank, rank) of this thread's points (at most 8 per thread, as in the spreading)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int p = (int)threadIdx.x + q * (int)blockDim.x;
+        key[q] = -1;
+        if (p >= sp.z) continue;
+        const int b = corners[sp.y + p] & 31;
+        key[q] = (b << 16) | atomicAdd(&cnt[b], 1);
+    }
     for (int s = 0; s < nvol; ++s)
         for (int r = threadIdx.x; r < tsize; r += blockDim.x) {
             const long gi = tile_cell_to_grid<DIM>(r, g, S);
             tile[s * tsize + r] = gi < 0 ? make_float2(0.f, 0.f) : __ldg(grid + (long)s * gstride + gi);
         }
     __syncthreads();
+    bank_table_fill(btab, cnt, sp.z);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        if (key[q] >= 0)
+            order[bank_position(btab, cnt, key[q] >> 16, key[q] & 0xffff)] =
+                (unsigned short)((int)threadIdx.x + q * (int)blockDim.x);
+    __syncthreads();
     const float inv_hw = 2.0f / (float)W;
-    for (int p = threadIdx.x; p < sp.z; p += blockDim.x) {
+    for (int k = threadIdx.x; k < sp.z; k += blockDim.x) {
+        const int p = order[k];
         const int j = perm[sp.y + p];
         PointInfo pi;
         point_at(pts, j, pi);
@@ -1270,9 +1328,10 @@ void NufftPlan::interp(Context &ctx, const float2 *grid, int nvol, float2 *c, Pt
     ProfScope ps(ctx, PS_INTERP, (double)nvol * (8.0 * pts_.M + 8.0 * gvol) + 4.0 * pts_.M);
     const size_t tile_bytes = (size_t)g.td[0] * g.td[1] * g.td[2] * sizeof(float2);
     int vchunk = (int)std::max<size_t>(1, (96 * 1024) / tile_bytes);
+    LC_REQUIRE(maxsub_ <= 8 * 256, "NUFFT interp: subproblem larger than the ordering pass");
     for (int v0 = 0; v0 < nvol; v0 += vchunk) {
         int nv = std::min(vchunk, nvol - v0);
-        size_t smem = tile_bytes * nv;
+        size_t smem = tile_bytes * nv + (size_t)maxsub_ * sizeof(unsigned short);
         const float2 *gv = grid + (long)v0 * gvol;
         float2 *cv = c + (long)v0 * pts_.M;
         dim3 gd(nsub_);
