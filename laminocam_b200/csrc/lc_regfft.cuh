@@ -221,6 +221,12 @@ struct RegPlan {
     X(1152, 9, 16, 8)    \
     X(1296, 9, 12, 12)
 
+// the odd ones
+#define LC_ODD_LINE_PLANS(X) \
+    X(81, 9, 3, 3)           \
+    X(243, 9, 9, 3)          \
+    X(729, 9, 9, 9)
+
 inline bool line_plan_exists(int M) {
     switch (M) {
 #define LC_LINE_HAS(m, r0, r1, r2) case m:
