@@ -108,21 +108,45 @@ static void gauss_legendre(int n, std::vector<double> &x, std::vector<double> &w
     }
 }
 
-std::vector<double> es_correction(int n, int nf, int w, double beta) {
+// Quadrature of the kernel's Fourier transform: Gauss-Legendre nodes x and
+// weights wt phi(x) on [-1, 1]
+static std::vector<double2> es_nodes(int w, double beta) {
     std::vector<double> x, wt;
     gauss_legendre(4 * w + 60, x, wt);
-    std::vector<double> phi(x.size());
-    for (size_t q = 0; q < x.size(); ++q) phi[q] = std::exp(beta * (std::sqrt(1.0 - x[q] * x[q]) - 1.0));
-    std::vector<double> out(n);
-    const double pi = 3.14159265358979323846;
-    for (int j = 0; j < n; ++j) {
-        double k = (double)(j - n / 2);
-        double xi = k * w * pi / nf;
-        double s = 0;
-        for (size_t q = 0; q < x.size(); ++q) s += wt[q] * phi[q] * std::cos(xi * x[q]);
-        out[j] = 2.0 / (w * s);
-    }
+    std::vector<double2> out(x.size());
+    for (size_t q = 0; q < x.size(); ++q)
+        out[q] = make_double2(x[q], wt[q] * std::exp(beta * (std::sqrt(1.0 - x[q] * x[q]) - 1.0)));
     return out;
+}
+
+// Deapodisation factors 2 / (w phihat(k w pi / nf)) of the n modes k = j - n/2,
+// one warp per mode, in FP64 (blocks of 128 threads).  (On the host the 76 to
+// 108 cosines per mode took 1 ms for 721 modes, five times per laminography
+// plan, with the device idle; one thread per mode took 25 us here.)
+__global__ void es_correction_kernel(const double2 *__restrict__ nodes, int nodes_n, int n, int nf, int w,
+                                     double *__restrict__ out, float *__restrict__ outf) {
+    const int j = (int)(blockIdx.x * 4 + (threadIdx.x >> 5)), lane = (int)(threadIdx.x & 31);
+    if (j >= n) return;
+    const double xi = (double)(j - n / 2) * w * 3.14159265358979323846 / nf;
+    double s = 0.0;
+    for (int q = lane; q < nodes_n; q += 32) {
+        const double2 p = nodes[q];
+        s += p.y * cos(xi * p.x);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+        const double c = 2.0 / (w * s);
+        out[j] = c;
+        outf[j] = (float)c;
+    }
+}
+
+// xy[y][x] = cy[y] cx[x]
+__global__ void outer_product_kernel(const double *__restrict__ cx, const double *__restrict__ cy, int nx, long n,
+                                     float *__restrict__ xy) {
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+        xy[i] = (float)(cy[i / nx] * cx[i % nx]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1153,20 +1177,24 @@ NufftPlan::NufftPlan(Context &ctx, const PolarGeometry &g, const int modes[3], d
         nb_[d] = (nf_[d] + bs_[d] - 1) / bs_[d];
     }
     cudaStream_t st = ctx.stream();
+    const std::vector<double2> nodes = es_nodes(w_, beta_);
+    DevBuf<double2> dnodes;
+    dnodes.upload(nodes.data(), nodes.size(), st);
+    DevBuf<double> cd[3];
     for (int d = 0; d < dim_; ++d) {
-        auto c = es_correction(modes_[d], nf_[d], w_, beta_);
-        std::vector<float> cf(c.begin(), c.end());
-        corr_[d].upload(cf.data(), cf.size(), st);
+        cd[d].alloc(modes_[d], st);
+        corr_[d].alloc(modes_[d], st);
+        es_correction_kernel<<<(modes_[d] + 3) / 4, 128, 0, st>>>(dnodes.get(), (int)nodes.size(), modes_[d], nf_[d],
+                                                                   w_, cd[d].get(), corr_[d].get());
+        LC_CHECK_LAUNCH();
     }
     if (dim_ == 3) {
-        auto cx_ = es_correction(modes_[0], nf_[0], w_, beta_);
-        auto cy_ = es_correction(modes_[1], nf_[1], w_, beta_);
-        std::vector<float> xy((size_t)modes_[0] * modes_[1]);
-        for (int y = 0; y < modes_[1]; ++y)
-            for (int x = 0; x < modes_[0]; ++x) xy[(size_t)y * modes_[0] + x] = (float)(cy_[y] * cx_[x]);
-        corr_xy_.upload(xy.data(), xy.size(), st);
+        const long n = (long)modes_[0] * modes_[1];
+        corr_xy_.alloc(n, st);
+        const long blocks = std::max<long>(1, std::min<long>((n + 255) / 256, (long)ctx.num_sms() * 8));
+        outer_product_kernel<<<(unsigned)blocks, 256, 0, st>>>(cd[0].get(), cd[1].get(), modes_[0], n, corr_xy_.get());
+        LC_CHECK_LAUNCH();
     }
-    LC_CUDA(cudaStreamSynchronize(st));
     sort_points(ctx);
 }
 
@@ -1196,25 +1224,17 @@ void NufftPlan::sort_points(Context &ctx) {
         acc += hc[b];
     }
     LC_REQUIRE(acc == pts_.Mh, "NUFFT: bin sort lost points");
-    // footprints over one cell: a footprint reaches at most w/2 + 1 <= bs
-    // cells beyond its point's cell, so only points of the bin and of its
-    // neighbours (wrapped, each counted once) can cover a cell of the bin;
-    // the neighbourhood sums are separable box sums of the bin counts
+    // Footprints over one cell: a footprint reaches at most w/2 + 1 <= bs cells
+    // beyond its point's cell, so only points of the bin and of its neighbours
+    // can cover a cell of the bin.  The bound sets the spacing between a bin's
+    // scale and the launch's 64-bit one (e_b <= e_G), which has bits to spare:
+    // the largest bin counted for every neighbour costs a few of them, and the
+    // exact sums over the neighbourhoods took 7 ms on the host for 135 k bins.
     {
-        std::vector<long> a(hc.begin(), hc.end()), t(nbins);
-        const long stride[3] = {1, nb_[0], (long)nb_[0] * nb_[1]};
-        for (int k = 0; k < 3; ++k) {
-            const int n = nb_[k];
-            const int lo = n >= 3 ? -1 : 0, hi = n >= 2 ? 1 : 0;  // distinct wrapped offsets
-            for (long b = 0; b < nbins; ++b) {
-                const int c = (int)((b / stride[k]) % n);
-                long sum = 0;
-                for (int d = lo; d <= hi; ++d) sum += a[b + (long)(((c + d + n) % n) - c) * stride[k]];
-                t[b] = sum;
-            }
-            a.swap(t);
-        }
-        kmax_ = std::max<long>(1, *std::max_element(a.begin(), a.end()));
+        long most = 1, neighbours = 1;
+        for (long b = 0; b < nbins; ++b) most = std::max<long>(most, hc[b]);
+        for (int k = 0; k < 3; ++k) neighbours *= std::min(nb_[k], 3);
+        kmax_ = std::max<long>(1, std::min(pts_.Mh, most * neighbours));
     }
     nsub_ = (int)subs.size();
     LC_REQUIRE(nsub_ > 0, "NUFFT: no points");

@@ -71,8 +71,6 @@ void geometry_init_3d(Context &ctx, PolarGeometry &g, const double *theta, const
 // kernel width and shape for a requested tolerance (upsampling factor 2)
 int es_width_for_tol(double tol);
 double es_beta_for_width(int w);
-// deapodisation factors 2/(w*phihat(k*w*pi/nf)) for the n modes k = j - n/2
-std::vector<double> es_correction(int n, int nf, int w, double beta);
 
 // Pointwise handling of the non-uniform values inside spread / interp.
 enum PtMode {
