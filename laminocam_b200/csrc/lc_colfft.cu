@@ -75,6 +75,7 @@ __device__ __forceinline__ void col_fft_body(const ColArgs &a, long bid) {
     float2 *tw = col_sm + NV * M * C;  // exp(-2 pi i m / M)
     float2 *th = tw + M;               // exp(-pi i m / M)
     load_line_twiddles<M>(tw);
+    chain_wait();
     const int c = threadIdx.x % C, t = threadIdx.x / C;
     const long o = bid / a.bpo;
     const long col = (bid - o * a.bpo) * C + c;
@@ -245,7 +246,7 @@ void launch_mode(cudaStream_t st, const ColArgs &a, long blocks) {
         LC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured.fetch_or(bit);
     }
-    kern<<<(unsigned)blocks, RegPlan<R0, R1, R2>::NT * kCols, smem, st>>>(a);
+    launch_chained(kern, (unsigned)blocks, RegPlan<R0, R1, R2>::NT * kCols, smem, st, a);
     LC_CHECK_LAUNCH();
 }
 

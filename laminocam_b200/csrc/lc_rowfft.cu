@@ -64,6 +64,7 @@ __device__ __forceinline__ void row_fft_body(const RowArgs &a, long bid) {
     float2 *tw = row_sm + M * kRowLines;  // exp(-2 pi i m / M)
     float2 *th = tw + M;                  // h(m) = exp(-pi i m / M)
     load_line_twiddles<M>(tw);
+    chain_wait();
     const int t = threadIdx.x % NT, c = threadIdx.x / NT;
     const long line = (bid * kRowLines + c) * row_reals(MODE);  // odd lengths: and line + 1
     const bool valid = line < a.n_lines;
@@ -305,7 +306,7 @@ void launch_row_mode(cudaStream_t st, const RowArgs &a, long blocks) {
         LC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured.fetch_or(bit);
     }
-    kern<<<(unsigned)blocks, RegPlan<R0, R1, R2>::NT * kRowLines, smem, st>>>(a);
+    launch_chained(kern, (unsigned)blocks, RegPlan<R0, R1, R2>::NT * kRowLines, smem, st, a);
     LC_CHECK_LAUNCH();
 }
 

@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(C *(A > B ? A : B))
         sincospif(2.0f * (float)m / (float)L, &s, &c);
         tw[m] = make_float2(c, -s);
     }
+    chain_wait();
     const int cl = threadIdx.x % C, j = threadIdx.x / C;
     const long col = (long)blockIdx.x * C + cl;
     const bool valid = col < n_inner;
@@ -154,6 +155,7 @@ template <int N>
 __global__ void __launch_bounds__(128, (N <= 32 ? 4 : 2))
     zdirect_kernel(float2 *data, long n_inner, int n, const float *__restrict__ taps) {
     const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    chain_wait();
     if (col >= n_inner) return;
     float2 x[N];
     float k[N];
@@ -180,7 +182,7 @@ template <int N>
 void launch_zd(cudaStream_t st, float2 *data, long n_inner, int n, const float *taps) {
     const long blocks = (n_inner + 127) / 128;
     LC_REQUIRE(blocks < (1L << 31), "direct z stage: grid too large");
-    zdirect_kernel<N><<<(unsigned)blocks, 128, 0, st>>>(data, n_inner, n, taps);
+    launch_chained(zdirect_kernel<N>, (unsigned)blocks, 128u, 0, st, data, n_inner, n, taps);
     LC_CHECK_LAUNCH();
 }
 
@@ -190,11 +192,11 @@ void launch_z(cudaStream_t st, float2 *data, long n_inner, int n_in, int n_out, 
     const long blocks = (n_inner + C - 1) / C;
     LC_REQUIRE(blocks < (1L << 31), "z convolution: grid too large");
     if (A % 2 == 0 && 2 * n_in <= A * B && 2 * n_out <= A * B)
-        zconv_kernel<A, B, C, (A % 2 == 0)><<<(unsigned)blocks, C * TPL, 0, st>>>(data, n_inner, n_in, n_out,
-                                                                                  spec, fold);
+        launch_chained(zconv_kernel<A, B, C, (A % 2 == 0)>, (unsigned)blocks, (unsigned)(C * TPL), 0, st, data,
+                       n_inner, n_in, n_out, spec, fold);
     else
-        zconv_kernel<A, B, C, false><<<(unsigned)blocks, C * TPL, 0, st>>>(data, n_inner, n_in, n_out, spec,
-                                                                          fold);
+        launch_chained(zconv_kernel<A, B, C, false>, (unsigned)blocks, (unsigned)(C * TPL), 0, st, data, n_inner,
+                       n_in, n_out, spec, fold);
     LC_CHECK_LAUNCH();
 }
 
