@@ -1,9 +1,11 @@
 // Bin-sorted ES-kernel spreading (type 1) and tile-staged interpolation
 // (type 2) on polar grids, plus the pruned fine-grid FFT passes.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <memory>
 #include <numeric>
+#include <unordered_map>
 
 #include "lc_nufft.hpp"
 
@@ -12,13 +14,80 @@ namespace lc {
 // ---------------------------------------------------------------------------
 // geometry
 // ---------------------------------------------------------------------------
-// one point of every pair of opposite lattice points
-static void set_lattice(PolarPts &p, int lat) {
+// One point of every pair of opposite lattice points, and one representative of
+// the angles with the same lattice.  axes: per angle the column axis (3 values)
+// and the row axis (3 values; zero in 2D).  Two angles match when their axes
+// agree up to sign after rounding to 1e-13 (k.x then differs by less than
+// 1e-9); a value on a rounding boundary only loses the saving.
+static void set_lattice(Context &ctx, PolarGeometry &g, int lat, const std::vector<double> &axes) {
+    PolarPts &p = g.pts;
+    using Key = std::array<long long, 6>;
+    struct Hash {
+        size_t operator()(const Key &k) const {
+            unsigned long long h = 0;
+            for (long long v : k) h = (h ^ (unsigned long long)v) * 0x9E3779B97F4A7C15ull;
+            return (size_t)(h ^ (h >> 32));
+        }
+    };
+    std::unordered_map<Key, int, Hash> seen(2 * (size_t)p.ntheta);
+    std::vector<std::vector<int2>> reps;
+    std::vector<std::array<int, 2>> sign0;  // signs of the representative's axes
+    for (int i = 0; i < p.ntheta; ++i) {
+        Key k{};
+        std::array<int, 2> sg{1, 1};
+        for (int v = 0; v < 2; ++v) {
+            long long q[3];
+            for (int d = 0; d < 3; ++d) q[d] = std::llround(axes[6 * (size_t)i + 3 * v + d] * 1e13);
+            const long long lead = q[0] != 0 ? q[0] : (q[1] != 0 ? q[1] : q[2]);
+            if (lead < 0) sg[v] = -1;
+            for (int d = 0; d < 3; ++d) k[3 * v + d] = sg[v] * q[d];
+        }
+        auto [it, fresh] = seen.emplace(k, (int)reps.size());
+        if (fresh) {
+            reps.emplace_back();
+            sign0.push_back(sg);
+        }
+        const std::array<int, 2> &s0 = sign0[it->second];
+        reps[it->second].push_back(make_int2(i, (sg[0] != s0[0] ? 1 : 0) | (sg[1] != s0[1] ? 2 : 0)));
+    }
+    std::vector<int> off{0};
+    std::vector<int2> mem;
+    for (const auto &r : reps) {
+        mem.insert(mem.end(), r.begin(), r.end());
+        off.push_back((int)mem.size());
+    }
+    if ((int)reps.size() == p.ntheta) {  // in the angles' own order
+        p.rcs = p.cs;
+        p.rrot = p.rot;
+    } else if (p.dim == 2) {
+        std::vector<double2> rcs;
+        for (const auto &r : reps)
+            rcs.push_back(make_double2(axes[6 * (size_t)r[0].x], axes[6 * (size_t)r[0].x + 1]));
+        g.rcs.upload(rcs.data(), rcs.size(), ctx.stream());
+        p.rcs = g.rcs.get();
+    } else {
+        std::vector<double> rr;
+        for (const auto &r : reps)
+            for (int d = 0; d < 3; ++d) {  // R00 R01 R10 R11 R20 R21
+                rr.push_back(axes[6 * (size_t)r[0].x + d]);
+                rr.push_back(axes[6 * (size_t)r[0].x + 3 + d]);
+            }
+        g.rrot.upload(rr.data(), rr.size(), ctx.stream());
+        p.rrot = g.rrot.get();
+    }
+    if (p.dim == 3 || (int)reps.size() < p.ntheta) {
+        g.moff.upload(off.data(), off.size(), ctx.stream());
+        g.mem.upload(mem.data(), mem.size(), ctx.stream());
+        p.moff = g.moff.get();
+        p.mem = g.mem.get();
+    }
+    p.nrep = (int)reps.size();
     p.lat = lat;
     p.half = (lat + 1) / 2;
     p.M = (long)p.ntheta * lat;
-    p.Mh = (long)p.ntheta * p.half;
+    p.Mh = (long)p.nrep * p.half;
     p.div_angle = make_fastdiv((unsigned)p.half);
+    LC_CUDA(cudaStreamSynchronize(ctx.stream()));
 }
 
 void geometry_init_2d(Context &ctx, PolarGeometry &g, const double *theta, int ntheta, int nr) {
@@ -28,13 +97,17 @@ void geometry_init_2d(Context &ctx, PolarGeometry &g, const double *theta, int n
     std::vector<double2> cs(ntheta);
     for (int i = 0; i < ntheta; ++i) cs[i] = make_double2(std::cos(theta[i]), std::sin(theta[i]));
     g.cs.upload(cs.data(), ntheta, ctx.stream());
-    LC_CUDA(cudaStreamSynchronize(ctx.stream()));
     g.pts = PolarPts{};
     g.pts.dim = 2;
     g.pts.ntheta = ntheta;
     g.pts.nr = nr;
     g.pts.cs = g.cs.get();
-    set_lattice(g.pts, nr);
+    std::vector<double> axes(6 * (size_t)ntheta, 0.0);
+    for (int i = 0; i < ntheta; ++i) {
+        axes[6 * (size_t)i] = cs[i].x;
+        axes[6 * (size_t)i + 1] = cs[i].y;
+    }
+    set_lattice(ctx, g, nr, axes);
 }
 
 void geometry_init_3d(Context &ctx, PolarGeometry &g, const double *theta, const double *gamma,
@@ -62,15 +135,20 @@ void geometry_init_3d(Context &ctx, PolarGeometry &g, const double *theta, const
     g.shifts.assign(2 * (size_t)ntheta, 0.0f);
     if (shifts) std::copy(shifts, shifts + 2 * (size_t)ntheta, g.shifts.begin());
     g.dshifts.upload(reinterpret_cast<const float2 *>(g.shifts.data()), ntheta, ctx.stream());
-    LC_CUDA(cudaStreamSynchronize(ctx.stream()));
     g.pts = PolarPts{};
     g.pts.dim = 3;
     g.pts.ntheta = ntheta;
     g.pts.nrows = nrows;
     g.pts.ncols = ncols;
     g.pts.rot = g.rot.get();
-    set_lattice(g.pts, nrows * ncols);
     g.pts.div_col = make_fastdiv((unsigned)ncols);
+    std::vector<double> axes(6 * (size_t)ntheta);
+    for (int i = 0; i < ntheta; ++i)
+        for (int d = 0; d < 3; ++d) {
+            axes[6 * (size_t)i + d] = rot[6 * (size_t)i + 2 * d];
+            axes[6 * (size_t)i + 3 + d] = rot[6 * (size_t)i + 2 * d + 1];
+        }
+    set_lattice(ctx, g, nrows * ncols, axes);
 }
 
 // ---------------------------------------------------------------------------
@@ -174,18 +252,18 @@ __device__ __forceinline__ unsigned fast_div(unsigned n, FastDiv f) { return (__
 struct PointInfo {
     double c[3];  // x, y, z
     double qX, qY;
-    int angle, l;  // angle and lattice point
-    bool flip;     // c is the negated coordinate
+    int l;      // lattice point
+    bool flip;  // c is the negated coordinate
 };
 
-// lattice point l of angle i
+// lattice point l of angle i (REP: of representative i)
+template <bool REP = false>
 __device__ __forceinline__ void lattice_point(const PolarPts &p, int i, int l, PointInfo &pi) {
-    pi.angle = i;
     pi.l = l;
     pi.flip = false;
     if (p.dim == 2) {
         double r = ((double)l + 0.5) * (2.0 * kPi / p.nr) - kPi;
-        double2 cs = p.cs[i];
+        const double2 cs = (REP ? p.rcs : p.cs)[i];
         pi.c[0] = cs.x * r;
         pi.c[1] = cs.y * r;
         pi.c[2] = 0.0;
@@ -196,7 +274,7 @@ __device__ __forceinline__ void lattice_point(const PolarPts &p, int i, int l, P
         const int a = (int)ua, b = l - (int)ua * p.ncols;
         double qX = ((double)b + 0.5) * (2.0 * kPi / p.ncols) - kPi;
         double qY = ((double)a + 0.5) * (2.0 * kPi / p.nrows) - kPi;
-        const double *R = p.rot + 6 * (long)i;
+        const double *R = (REP ? p.rrot : p.rot) + 6 * (long)i;
         pi.c[0] = R[0] * qX + R[1] * qY;
         pi.c[1] = R[2] * qX + R[3] * qY;
         pi.c[2] = R[4] * qX + R[5] * qY;
@@ -205,14 +283,15 @@ __device__ __forceinline__ void lattice_point(const PolarPts &p, int i, int l, P
     }
 }
 
-// Folded point j: one of each pair of opposite lattice points, negated when
+// Folded point j: one of each pair of opposite lattice points of a representative
+// angle, negated when
 // its y coordinate (wrapped to [-pi, pi]) is below zero, so that the folded
 // points fill the half of the fine grid with y >= 0 at the density of the
 // full set.
 __device__ __forceinline__ void point_at(const PolarPts &p, long j, PointInfo &pi) {
     const unsigned jj = (unsigned)j;  // below 2^31
-    const unsigned i = fast_div(jj, p.div_angle);
-    lattice_point(p, (int)i, (int)(jj - i * (unsigned)p.half), pi);
+    const unsigned r = fast_div(jj, p.div_angle);
+    lattice_point<true>(p, (int)r, (int)(jj - r * (unsigned)p.half), pi);
     if (pi.c[1] - 2.0 * kPi * rint(pi.c[1] * kInv2Pi) < 0.0) {
         pi.flip = true;
 #pragma unroll
@@ -224,36 +303,133 @@ __device__ __forceinline__ bool in_band(const PointInfo &pi) {
     return fabs(pi.c[0]) <= kPi && fabs(pi.c[1]) <= kPi && fabs(pi.c[2]) <= kPi;
 }
 
-// Band flags kept in the upper bits of a sorted point's corner: the point and
-// its opposite are tested separately (rounding decides for a lattice point on
-// the boundary).
-constexpr unsigned kCornerMask = 0x3fffu, kOutOwn = 0x8000u, kOutOpp = 0x4000u;
+// Kept in the upper bit of a sorted point's corner: every lattice point that
+// the folded point stands for is outside the band.
+constexpr unsigned kCornerMask = 0x7fffu, kOut = 0x8000u;
+
+// lattice point of a member angle that coincides with point l of its
+// representative (flips: bit 0 columns or radius, bit 1 rows)
+__device__ __forceinline__ int member_point(const PolarPts &p, int l, int flips) {
+    if (flips == 0) return l;
+    if (p.dim == 2) return p.lat - 1 - l;
+    const int a = (int)fast_div((unsigned)l, p.div_col), b = l - a * p.ncols;
+    return (flips & 2 ? p.nrows - 1 - a : a) * p.ncols + (flips & 1 ? p.ncols - 1 - b : b);
+}
+
+__device__ __forceinline__ bool point_in_band(const PolarPts &p, int angle, int l) {
+    PointInfo pi;
+    lattice_point(p, angle, l, pi);
+    return in_band(pi);
+}
 
 // Type 1 keeps the real part of sum_j c_j exp(i k.x_j).  The pair x, -x adds
 //   Re(c e^{i k.x} + c' e^{-i k.x}) = Re((c + conj c') e^{i k.x}),
 // so one point with the value c + conj(c') stands for both (its conjugate
-// when the point is negated), at half the footprints to spread: the 3D
-// spreading of 360 x 511 x 511 values onto 48 x 1024 x 1024 cells took 14.3 ms
-// with every point and 7.1 ms folded.  Values outside the band are left out;
-// cv is the volume's value array, out the flags that count.  herm: c' = conj c
-// is known and not read.
-__device__ __forceinline__ float2 fold_value(const PolarPts &p, const float2 *__restrict__ cv, int angle, int l,
-                                             unsigned out, bool herm) {
-    const float2 *a = cv + (long)angle * p.lat;
-    float2 v = make_float2(0.f, 0.f);
-    if (herm) {
-        const float2 w = a[l];
-        float f = (out & kOutOwn) ? 0.f : 1.f;
-        if (2 * l + 1 != p.lat && !(out & kOutOpp)) f += 1.f;
-        return make_float2(f * w.x, f * w.y);
+// when the point is negated), and the members of a representative angle, whose
+// points coincide, add up.  This pass forms the folded values, with the band
+// limit (rounding decides for a lattice point on the boundary, so every point
+// is tested on its own) and the phases of the shifts; the sort, the bounds and
+// the spreading then work on nrep * half points instead of ntheta * lat.
+// Spreading 360 x 511 x 511 values over a full turn onto 48 x 1024 x 1024
+// cells: 14.3 ms with every point, 7.0 ms with one of each opposite pair, 3.7 ms with
+// one of each pair of opposite angles, and 0.4 ms for this pass.
+// herm: c' = conj c is known, and only lattice points below half are read.
+__global__ void __launch_bounds__(256) fold_values_kernel(PolarPts pts, const float2 *__restrict__ c, int nvol,
+                                                          int mode, int herm, const float2 *__restrict__ shifts,
+                                                          float2 *__restrict__ vals) {
+    const bool band = mode != PT_PLAIN && pts.dim == 3;
+    for (long j = (long)blockIdx.x * blockDim.x + threadIdx.x; j < pts.Mh; j += (long)gridDim.x * blockDim.x) {
+        PointInfo pi;
+        point_at(pts, j, pi);
+        const int r = (int)fast_div((unsigned)j, pts.div_angle);
+        const int m0 = pts.moff[r], m1 = pts.moff[r + 1];
+        for (int s = 0; s < nvol; ++s) {
+            float2 v = make_float2(0.f, 0.f);
+            for (int m = m0; m < m1; ++m) {
+                const int2 mb = pts.mem[m];
+                const int l = member_point(pts, pi.l, mb.y), o = pts.lat - 1 - l;
+                const bool in_l = !band || point_in_band(pts, mb.x, l);
+                const bool in_o = l != o && (!band || point_in_band(pts, mb.x, o));
+                const float2 *a = c + (long)s * pts.M + (long)mb.x * pts.lat;
+                float2 t = make_float2(0.f, 0.f);
+                if (herm) {
+                    const float2 w = a[l < o ? l : o];
+                    const float f = (in_l ? 1.f : 0.f) + (in_o ? 1.f : 0.f);
+                    t = make_float2(f * w.x, l > o ? -f * w.y : f * w.y);
+                } else {
+                    if (in_l) t = a[l];
+                    if (in_o) {
+                        const float2 w = a[o];
+                        t.x += w.x;
+                        t.y -= w.y;
+                    }
+                }
+                if (mode == PT_SHIFT) {
+                    PointInfo pm;
+                    lattice_point(pts, mb.x, l, pm);
+                    const float2 sh = shifts[mb.x];
+                    double sn, cs;
+                    sincos(pm.qX * (double)sh.x + pm.qY * (double)sh.y, &sn, &cs);
+                    t = cmul(t, make_float2((float)cs, (float)-sn));
+                }
+                v = cadd(v, t);
+            }
+            if (pi.flip) v.y = -v.y;
+            vals[(long)s * pts.Mh + j] = v;
+        }
     }
-    if (!(out & kOutOwn)) v = a[l];
-    if (2 * l + 1 != p.lat && !(out & kOutOpp)) {
+}
+
+// In 2D, where no two angles share a lattice, the spreading and the
+// interpolation read and write the lattice values themselves: the two passes
+// would cost more than they save (four 511^2 slices: projection 103 -> 108 us,
+// four 1023^2 slices: backprojection 439 -> 453 us with them).
+struct Direct2D {
+    int on;    // the values are the lattice's, [nvol][M], not folded ones
+    int herm;  // type 1: opposite values are conjugates, only l < half is stored
+    int keep;  // type 2: lattice points stored
+};
+
+// folded value of point j (angle i, lattice point l), up to the sign of its
+// imaginary part when the point is negated
+__device__ __forceinline__ float2 direct_value(const PolarPts &p, const float2 *__restrict__ c, int i, int l,
+                                               int herm) {
+    const float2 *a = c + (long)i * p.lat;
+    float2 v = a[l];
+    if (2 * l + 1 != p.lat) {
+        if (herm) return make_float2(2.f * v.x, 2.f * v.y);
         const float2 w = a[p.lat - 1 - l];
         v.x += w.x;
         v.y -= w.y;
     }
     return v;
+}
+
+// Type 2 of a real volume has C(-x) = conj C(x): the value at a folded point
+// goes to both lattice points of the pair, in every member angle (zero outside
+// the band; only lattice points below keep are stored).
+__global__ void __launch_bounds__(256) expand_values_kernel(PolarPts pts, const float2 *__restrict__ vals, int nvol,
+                                                            int mode, int keep, float2 *__restrict__ c) {
+    const bool band = mode != PT_PLAIN && pts.dim == 3;
+    const float2 zero = make_float2(0.f, 0.f);
+    for (long j = (long)blockIdx.x * blockDim.x + threadIdx.x; j < pts.Mh; j += (long)gridDim.x * blockDim.x) {
+        PointInfo pi;
+        point_at(pts, j, pi);
+        const int r = (int)fast_div((unsigned)j, pts.div_angle);
+        for (int m = pts.moff[r]; m < pts.moff[r + 1]; ++m) {
+            const int2 mb = pts.mem[m];
+            const int l = member_point(pts, pi.l, mb.y), o = pts.lat - 1 - l;
+            const bool st_l = l < keep, st_o = o != l && o < keep;
+            const bool in_l = !band || point_in_band(pts, mb.x, l), in_o = !band || point_in_band(pts, mb.x, o);
+            float2 *a = c + (long)mb.x * pts.lat;
+            for (int s = 0; s < nvol; ++s) {
+                float2 v = vals[(long)s * pts.Mh + j];
+                if (pi.flip) v.y = -v.y;
+                if (st_l) a[(long)s * pts.M + l] = in_l ? v : zero;
+                if (st_o) a[(long)s * pts.M + o] = in_o ? cconj(v) : zero;
+            }
+        }
+    }
 }
 
 // wrapped fine-grid coordinate u in [0, nf), its cell, first covered cell l0
@@ -348,7 +524,7 @@ __device__ __forceinline__ int bin_corner_of(const PointInfo &pi, const GridCfg 
 
 // perm[k] = the folded point at sorted position k; corners[k] its footprint
 // corner in its bin's tile (read by the footprint bound and the spreading's
-// bucketing) and its band flags
+// bucketing) and its band flag
 template <int DIM>
 __global__ void bin_scatter_kernel(PolarPts pts, GridCfg g, int W, int *cursor, int *perm,
                                    unsigned short *corners) {
@@ -359,10 +535,14 @@ __global__ void bin_scatter_kernel(PolarPts pts, GridCfg g, int W, int *cursor, 
         int corner;
         int b = bin_corner_of<DIM>(pi, g, W, corner);
         if (DIM == 3) {
-            if (!in_band(pi)) corner |= (int)kOutOwn;
-            PointInfo po;
-            lattice_point(pts, pi.angle, pts.lat - 1 - pi.l, po);
-            if (!in_band(po)) corner |= (int)kOutOpp;
+            bool in = false;
+            const unsigned rp = fast_div((unsigned)j, pts.div_angle);
+            for (int m = pts.moff[rp]; m < pts.moff[rp + 1] && !in; ++m) {
+                const int2 mb = pts.mem[m];
+                const int l = member_point(pts, pi.l, mb.y);
+                in = point_in_band(pts, mb.x, l) || point_in_band(pts, mb.x, pts.lat - 1 - l);
+            }
+            if (!in) corner |= (int)kOut;
         }
         unsigned act = __activemask();
         unsigned peers = __match_any_sync(act, b);
@@ -570,29 +750,19 @@ __device__ __forceinline__ void rot_banks(int rot, int plane, int &d1, int &d2) 
     d2 = (plane * (rot - W)) & 31;
 }
 
-// Spreads the folded point j (cf: its corner and band flags); in 3D its footprint planes are visited in the order rotated
+// Spreads the folded point j (cf: its corner and band flag); in 3D its footprint planes are visited in the order rotated
 // by rot (0: in order).
 template <int DIM, int W>
 __device__ __forceinline__ void spread_point(const PolarPts &pts, const GridCfg &g,
-                                             const float2 *__restrict__ c, int nvol, int j, unsigned cf,
-                                             int mode, bool herm, const float2 *__restrict__ shifts,
-                                             int tx, int plane, int tsize, unsigned sm_re,
+                                             const float2 *__restrict__ vals, Direct2D dir, int nvol, int j,
+                                             unsigned cf, int tx, int plane, int tsize, unsigned sm_re,
                                              unsigned plane_bytes, float fscale, int rot) {
     const float inv_hw = 2.0f / (float)W;
     PointInfo pi;
     point_at(pts, j, pi);
-    float2 mult = make_float2(fscale, 0.f);
-    if (mode == PT_SHIFT) {
-        const float2 sh = shifts[pi.angle];
-        const double ph = pi.qX * (double)sh.x + pi.qY * (double)sh.y;
-        double sn, cs;
-        sincos(ph, &sn, &cs);
-        mult = make_float2((float)cs * fscale, (float)-sn * fscale);
-    }
     // wk[d][m]: weight of the cell at offset m along axis d (3D z: (m + rot) mod W)
     float wk[DIM][W];
     const int corner = (int)(cf & kCornerMask);
-    const unsigned out = mode == PT_PLAIN ? 0u : cf;
     {
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
@@ -609,9 +779,14 @@ __device__ __forceinline__ void spread_point(const PolarPts &pts, const GridCfg 
         }
     }
     for (int s = 0; s < nvol; ++s) {
-        float2 v = fold_value(pts, c + (long)s * pts.M, pi.angle, pi.l, out, herm);
-        v = mode == PT_SHIFT ? cmul(v, mult) : make_float2(v.x * fscale, v.y * fscale);
-        if (pi.flip) v.y = -v.y;
+        float2 v;
+        if (DIM == 2 && dir.on) {
+            v = direct_value(pts, vals + (long)s * pts.M, (int)fast_div((unsigned)j, pts.div_angle), pi.l, dir.herm);
+            if (pi.flip) v.y = -v.y;
+        } else {
+            v = vals[(long)s * pts.Mh + j];
+        }
+        v = make_float2(v.x * fscale, v.y * fscale);
         // 32-bit shared addresses of the footprint corner in the two planes
         const unsigned ar = sm_re + 4u * (unsigned)(s * tsize + corner);
         const unsigned ai = ar + plane_bytes;
@@ -714,23 +889,21 @@ __global__ void __launch_bounds__(256) bin_footprint_kernel(GridCfg g, OffsetWei
 // the bin's points (one CTA per subproblem), and their maximum over the launch,
 // as the bits of non-negative floats (integer order equals float order; binm
 // and mbits zeroed first)
-__global__ void __launch_bounds__(256) bin_value_bound_kernel(PolarPts pts, const float2 *__restrict__ c,
-                                                              int nvol, const int *__restrict__ perm,
-                                                              const unsigned short *__restrict__ corners,
-                                                              const int4 *__restrict__ subs, int mode, int herm,
-                                                              int *binm, int *mbits) {
+__global__ void __launch_bounds__(256) bin_value_bound_kernel(PolarPts pts, const float2 *__restrict__ vals,
+                                                              Direct2D dir, int nvol, const int *__restrict__ perm,
+                                                              const int4 *__restrict__ subs, int *binm, int *mbits) {
     __shared__ int mx;
     const int4 sp = subs[blockIdx.x];
     if (threadIdx.x == 0) mx = 0;
     __syncthreads();
     float m = 0.f;
+#pragma unroll 4
     for (int p = threadIdx.x; p < sp.z; p += blockDim.x) {
-        const unsigned j = (unsigned)perm[sp.y + p];
-        const unsigned i = fast_div(j, pts.div_angle);
-        const unsigned out = mode == PT_PLAIN ? 0u : corners[sp.y + p];
+        const int j = perm[sp.y + p];
+        const int i = (int)fast_div((unsigned)j, pts.div_angle);
         for (int s = 0; s < nvol; ++s) {
-            const float2 v = fold_value(pts, c + (long)s * pts.M, (int)i, (int)(j - i * (unsigned)pts.half), out,
-                                        herm != 0);
+            const float2 v = dir.on ? direct_value(pts, vals + (long)s * pts.M, i, j - i * pts.half, dir.herm)
+                                    : vals[(long)s * pts.Mh + j];
             m = fmaxf(m, fabsf(v.x) + fabsf(v.y));
         }
     }
@@ -750,12 +923,11 @@ __global__ void __launch_bounds__(256) bin_value_bound_kernel(PolarPts pts, cons
 
 template <int DIM, int W>
 __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
-    spread_kernel(PolarPts pts, GridCfg g, const float2 *__restrict__ c, int nvol,
+    spread_kernel(PolarPts pts, GridCfg g, const float2 *__restrict__ vals, Direct2D dir, int nvol,
                   const int *__restrict__ perm, const unsigned short *__restrict__ corners,
                   const int4 *__restrict__ subs,
-                  unsigned long long *__restrict__ fix, long gstride, int mode, int herm,
-                  const float2 *__restrict__ shifts, const int *__restrict__ mbits, long kmax,
-                  const int *__restrict__ kbin, const int *__restrict__ binm) {
+                  unsigned long long *__restrict__ fix, long gstride, int mode, const int *__restrict__ mbits,
+                  long kmax, const int *__restrict__ kbin, const int *__restrict__ binm) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int cnt[32], start[32], mincnt, maxcnt;
     __shared__ BankTable btab;  // 2D
@@ -795,7 +967,7 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
         if (p >= sp.z) continue;
         int k = -1;
         const unsigned cf = corners[sp.y + p];  // from the bin sort
-        if (mode == PT_PLAIN || (cf & (kOutOwn | kOutOpp)) != (kOutOwn | kOutOpp)) {
+        if (mode == PT_PLAIN || !(cf & kOut)) {
             const int corner = (int)(cf & kCornerMask);
             const int b = corner & 31;
             k = (b << 16) | atomicAdd(&cnt[b], 1);
@@ -908,8 +1080,8 @@ __global__ void __launch_bounds__(kSpreadThreads, LC_SPREAD_MIN_BLOCKS)
             }
         }
         if (p >= 0)
-            spread_point<DIM, W>(pts, g, c, nvol, perm[sp.y + p], corners[sp.y + p], mode, herm != 0, shifts,
-                                 tx, plane, tsize, sm_re, plane_bytes, fscale, prot);
+            spread_point<DIM, W>(pts, g, vals, dir, nvol, perm[sp.y + p], corners[sp.y + p], tx, plane, tsize, sm_re,
+                                 plane_bytes, fscale, prot);
     }
     __syncthreads();
     // flush the tile's exact sums at the launch's scale (halos overlap
@@ -946,8 +1118,8 @@ __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
                                                      const float2 *__restrict__ grid, long gstride,
                                                      int nvol, const int *__restrict__ perm,
                                                      const unsigned short *__restrict__ corners,
-                                                     const int4 *__restrict__ subs, float2 *__restrict__ c,
-                                                     int mode, int keep) {
+                                                     const int4 *__restrict__ subs, float2 *__restrict__ vals,
+                                                     Direct2D dir, int mode) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int cnt[32];
     __shared__ BankTable btab;
@@ -1000,19 +1172,7 @@ __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
         const int j = perm[sp.y + p];
         PointInfo pi;
         point_at(pts, j, pi);
-        const unsigned out = mode == PT_PLAIN ? 0u : corners[sp.y + p];
-        // a real volume has C(-x) = conj C(x): the point's value is stored at
-        // both lattice points of the pair (zero outside the band)
-        float2 *own = c + (long)pi.angle * pts.lat + pi.l;
-        float2 *opp = c + (long)pi.angle * pts.lat + (pts.lat - 1 - pi.l);
-        const bool both = own != opp && pts.lat - 1 - pi.l < keep;
-        if ((out & (kOutOwn | kOutOpp)) == (kOutOwn | kOutOpp)) {
-            for (int s = 0; s < nvol; ++s) {
-                own[(long)s * pts.M] = make_float2(0.f, 0.f);
-                if (both) opp[(long)s * pts.M] = make_float2(0.f, 0.f);
-            }
-            continue;
-        }
+        if (mode != PT_PLAIN && (corners[sp.y + p] & kOut)) continue;  // stored as zero by the expansion
         float wk[2][W];
         int lo[3] = {0, 0, 0};
         float offz = 0.f;
@@ -1067,23 +1227,29 @@ __global__ void __launch_bounds__(256) interp_kernel(PolarPts pts, GridCfg g,
                     ai = fmaf(zi, wz, ai);
                 }
             }
-            if (pi.flip) ai = -ai;
-            own[(long)s * pts.M] = (out & kOutOwn) ? make_float2(0.f, 0.f) : make_float2(ar, ai);
-            if (both) opp[(long)s * pts.M] = (out & kOutOpp) ? make_float2(0.f, 0.f) : make_float2(ar, -ai);
+            if (DIM == 2 && dir.on) {
+                float2 *a = vals + (long)s * pts.M + (long)fast_div((unsigned)j, pts.div_angle) * pts.lat;
+                const int o = pts.lat - 1 - pi.l;
+                if (pi.flip) ai = -ai;
+                a[pi.l] = make_float2(ar, ai);
+                if (o != pi.l && o < dir.keep) a[o] = make_float2(ar, -ai);
+            } else {
+                vals[(long)s * pts.Mh + j] = make_float2(ar, ai);
+            }
         }
     }
 }
 
 template <int DIM, int W>
 void launch_spread_w(const Context &ctx, dim3 grid, size_t smem, cudaStream_t st, const PolarPts &pts,
-                     const GridCfg &g, const float2 *c, int nvol, const int *perm,
+                     const GridCfg &g, const float2 *vals, const Direct2D &dir, int nvol, const int *perm,
                      const unsigned short *corners, const int4 *subs, unsigned long long *out, long gstride,
-                     int mode, int herm, const float2 *shifts, const int *mbits, long kmax, const int *kbin,
+                     int mode, const int *mbits, long kmax, const int *kbin,
                      const int *binm) {
     auto kern = spread_kernel<DIM, W>;
     allow_max_dynamic_smem(ctx, kern);
-    kern<<<grid, kSpreadThreads, smem, st>>>(pts, g, c, nvol, perm, corners, subs, out, gstride,
-                                             mode, herm, shifts, mbits, kmax, kbin, binm);
+    kern<<<grid, kSpreadThreads, smem, st>>>(pts, g, vals, dir, nvol, perm, corners, subs, out, gstride,
+                                             mode, mbits, kmax, kbin, binm);
     LC_CHECK_LAUNCH();
 }
 
@@ -1099,10 +1265,10 @@ void launch_footprint_w(const Context &ctx, unsigned nbins, size_t smem, cudaStr
 template <int DIM, int W>
 void launch_interp_w(const Context &ctx, dim3 grid, int threads, size_t smem, cudaStream_t st,
                      const PolarPts &pts, const GridCfg &g, const float2 *gr, long gstride, int nvol,
-                     const int *perm, const unsigned short *corners, const int4 *subs, float2 *c, int mode, int keep) {
+                     const int *perm, const unsigned short *corners, const int4 *subs, float2 *vals, const Direct2D &dir, int mode) {
     auto kern = interp_kernel<DIM, W>;
     allow_max_dynamic_smem(ctx, kern);
-    kern<<<grid, threads, smem, st>>>(pts, g, gr, gstride, nvol, perm, corners, subs, c, mode, keep);
+    kern<<<grid, threads, smem, st>>>(pts, g, gr, gstride, nvol, perm, corners, subs, vals, dir, mode);
     LC_CHECK_LAUNCH();
 }
 
@@ -1306,12 +1472,23 @@ void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, Pt
     LC_CUDA(cudaMemsetAsync(fix_.get(), 0, 2 * gvol * nvol * sizeof(long long), st));
     const int vchunk = (int)std::max<size_t>(1, (96 * 1024) / tile_bytes);
     const long nbins = (long)nb_[0] * nb_[1] * nb_[2];
+    const Direct2D dir{dim_ == 2 && pts_.nrep == pts_.ntheta ? 1 : 0, herm ? 1 : 0, 0};
+    const float2 *vals = c;
+    long vstride = pts_.M;
+    if (!dir.on) {
+        vals_.ensure((long)nvol * pts_.Mh, st);
+        vals = vals_.get();
+        vstride = pts_.Mh;
+        const long blocks = std::max<long>(1, std::min<long>((pts_.Mh + 255) / 256, (long)ctx.num_sms() * 32));
+        fold_values_kernel<<<(unsigned)blocks, 256, 0, st>>>(pts_, c, nvol, mode, herm ? 1 : 0, shifts_, vals_.get());
+        LC_CHECK_LAUNCH();
+    }
     // the bins' value bounds per chunk of volumes, and the launch's
     binm_.ensure(nbins * ((nvol + vchunk - 1) / vchunk), st);
     LC_CUDA(cudaMemsetAsync(binm_.get(), 0, binm_.size() * sizeof(int), st));
     for (int v0 = 0; v0 < nvol; v0 += vchunk) {
-        bin_value_bound_kernel<<<nsub_, 256, 0, st>>>(pts_, c + (long)v0 * pts_.M, std::min(vchunk, nvol - v0),
-                                                      perm_.get(), corner_.get(), subs_.get(), mode, herm ? 1 : 0,
+        bin_value_bound_kernel<<<nsub_, 256, 0, st>>>(pts_, vals + (long)v0 * vstride, dir,
+                                                      std::min(vchunk, nvol - v0), perm_.get(), subs_.get(),
                                                       binm_.get() + nbins * (v0 / vchunk), mbits_.get());
         LC_CHECK_LAUNCH();
     }
@@ -1320,18 +1497,16 @@ void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, Pt
         const int nv = std::min(vchunk, nvol - v0);
         const size_t smem = tile_bytes * nv + bucket_bytes;
         LC_REQUIRE(smem <= ctx.max_smem(), "NUFFT spread: tile does not fit shared memory");
-        const float2 *cv = c + (long)v0 * pts_.M;
+        const float2 *cv = vals + (long)v0 * vstride;
         unsigned long long *fv = fix + 2 * (long)v0 * gvol;
         dim3 gd(nsub_);
         const int *bm = binm_.get() + nbins * (v0 / vchunk);
         if (dim_ == 2) {
-            LC_W_SWITCH(w_, (launch_spread_w<2, WW>(ctx, gd, smem, st, pts_, g, cv, nv,
-                                                   perm_.get(), corner_.get(), subs_.get(), fv, gvol, mode, herm ? 1 : 0, shifts_,
-                                                   mbits_.get(), kmax_, kbin_.get(), bm)));
+            LC_W_SWITCH(w_, (launch_spread_w<2, WW>(ctx, gd, smem, st, pts_, g, cv, dir, nv,
+                                                   perm_.get(), corner_.get(), subs_.get(), fv, gvol, mode, mbits_.get(), kmax_, kbin_.get(), bm)));
         } else {
-            LC_W_SWITCH(w_, (launch_spread_w<3, WW>(ctx, gd, smem, st, pts_, g, cv, nv,
-                                                   perm_.get(), corner_.get(), subs_.get(), fv, gvol, mode, herm ? 1 : 0, shifts_,
-                                                   mbits_.get(), kmax_, kbin_.get(), bm)));
+            LC_W_SWITCH(w_, (launch_spread_w<3, WW>(ctx, gd, smem, st, pts_, g, cv, dir, nv,
+                                                   perm_.get(), corner_.get(), subs_.get(), fv, gvol, mode, mbits_.get(), kmax_, kbin_.get(), bm)));
         }
     }
     {
@@ -1347,22 +1522,28 @@ void NufftPlan::interp(Context &ctx, const float2 *grid, int nvol, float2 *c, Pt
     const long gvol = (long)nf_[0] * ny_ * nf_[2];
     ProfScope ps(ctx, PS_INTERP, (double)nvol * (8.0 * pts_.M + 8.0 * gvol) + 4.0 * pts_.M);
     const size_t tile_bytes = (size_t)g.td[0] * g.td[1] * g.td[2] * sizeof(float2);
+    const Direct2D dir{dim_ == 2 && pts_.nrep == pts_.ntheta ? 1 : 0, 0, keep};
+    if (!dir.on) vals_.ensure((long)nvol * pts_.Mh, ctx.stream());
     int vchunk = (int)std::max<size_t>(1, (96 * 1024) / tile_bytes);
     LC_REQUIRE(maxsub_ <= 8 * 256, "NUFFT interp: subproblem larger than the ordering pass");
     for (int v0 = 0; v0 < nvol; v0 += vchunk) {
         int nv = std::min(vchunk, nvol - v0);
         size_t smem = tile_bytes * nv + (size_t)maxsub_ * sizeof(unsigned short);
         const float2 *gv = grid + (long)v0 * gvol;
-        float2 *cv = c + (long)v0 * pts_.M;
+        float2 *cv = dir.on ? c + (long)v0 * pts_.M : vals_.get() + (long)v0 * pts_.Mh;
         dim3 gd(nsub_);
         if (dim_ == 2) {
             LC_W_SWITCH(w_, (launch_interp_w<2, WW>(ctx, gd, 256, smem, ctx.stream(), pts_, g, gv, gvol, nv,
-                                                   perm_.get(), corner_.get(), subs_.get(), cv, mode, keep)));
+                                                   perm_.get(), corner_.get(), subs_.get(), cv, dir, mode)));
         } else {
             LC_W_SWITCH(w_, (launch_interp_w<3, WW>(ctx, gd, 256, smem, ctx.stream(), pts_, g, gv, gvol, nv,
-                                                   perm_.get(), corner_.get(), subs_.get(), cv, mode, keep)));
+                                                   perm_.get(), corner_.get(), subs_.get(), cv, dir, mode)));
         }
     }
+    if (dir.on) return;
+    const long blocks = std::max<long>(1, std::min<long>((pts_.Mh + 255) / 256, (long)ctx.num_sms() * 32));
+    expand_values_kernel<<<(unsigned)blocks, 256, 0, ctx.stream()>>>(pts_, vals_.get(), nvol, mode, keep, c);
+    LC_CHECK_LAUNCH();
 }
 
 void NufftPlan::type1_real(Context &ctx, const float2 *c, int nvol, float *out, float scale,

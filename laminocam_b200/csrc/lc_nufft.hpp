@@ -47,11 +47,20 @@ struct PolarPts {
     const double *rot = nullptr;  // R00 R01 R10 R11 R20 R21 per angle
     // The lattice of an angle (lat = nr points in 2D, nrows * ncols in 3D) is
     // closed under negation: lattice point l and lat - 1 - l are opposite.  A
-    // plan handles one point of each pair: half = ceil(lat / 2) per angle,
-    // l < half, Mh over all angles (see fold_value).
-    int lat = 0, half = 0;
+    // plan handles one point of each pair, half = ceil(lat / 2) per angle,
+    // l < half.  Angles whose lattices hold the same points (axes equal up to
+    // sign: theta and theta + 180 degrees of a full turn) share one
+    // representative: nrep of them, Mh = nrep * half folded points in all.
+    // Members of representative r: mem[moff[r] .. moff[r + 1]), the angle and
+    // the flips that map the representative's lattice onto the member's (bit
+    // 0: columns, or the radius in 2D; bit 1: rows).
+    int lat = 0, half = 0, nrep = 0;
     long Mh = 0;
-    // folded point index -> angle (by half) and, in 3D, lattice point -> row (by ncols)
+    const int *moff = nullptr;
+    const int2 *mem = nullptr;  // the first member is the representative, unflipped
+    const double2 *rcs = nullptr;  // cs and rot of the representatives
+    const double *rrot = nullptr;
+    // folded point index -> representative (by half) and, in 3D, lattice point -> row (by ncols)
     FastDiv div_angle, div_col;
 };
 
@@ -62,6 +71,10 @@ struct PolarGeometry {
     DevBuf<double2> cs;
     DevBuf<double> rot;
     DevBuf<float2> dshifts;
+    DevBuf<int> moff;
+    DevBuf<int2> mem;
+    DevBuf<double2> rcs;
+    DevBuf<double> rrot;
 };
 
 void geometry_init_2d(Context &ctx, PolarGeometry &g, const double *theta, int ntheta, int nr);
@@ -85,7 +98,7 @@ class NufftPlan {
     NufftPlan(Context &ctx, const PolarGeometry &g, const int modes[3], double tol);
     // type 1: c [nvol][M] complex -> out real [nvol][n1][n2][n3] = Re(f) * scale.
     // herm: the values at opposite lattice points are conjugates; only lattice
-    // points below half are read.
+    // points below half are read.  (Any plan geometry; see fold_values_kernel.)
     void type1_real(Context &ctx, const float2 *c, int nvol, float *out, float scale,
                     PtMode mode, bool herm = false);
     // type 2: real in [nvol][...modes] -> c [nvol][M].  keep > 0: only lattice
@@ -115,7 +128,8 @@ class NufftPlan {
     DevBuf<float> corr_[3];
     DevBuf<float> corr_xy_;  // corr_y (x) corr_x, 3D type 2
     DevBuf<int> perm_;
-    DevBuf<unsigned short> corner_;  // per sorted point: footprint corner in its bin's tile, band flags
+    DevBuf<unsigned short> corner_;  // per sorted point: footprint corner in its bin's tile, band flag
+    DevBuf<float2> vals_;            // folded values, [nvol][Mh]
     DevBuf<int4> subs_;
     int nsub_ = 0;
     int maxsub_ = 1024;  // most points of one spreading subproblem

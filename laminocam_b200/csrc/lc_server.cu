@@ -200,7 +200,9 @@ size_t estimate_bytes(const Job &j) {
     const size_t nt = j.d0, M = nt * PR * PC, nv = (size_t)N[0] * N[1] * N[2];
     const size_t fine = next23(2 * N[0]) * next23(2 * N[1]) * next23(2 * N[2]);
     size_t b = 4 * nt * j.d1 * j.d2 + 4 * M + 8 * M;  // raw and padded projections, complex lines
-    b += 4 * M + 3 * 8 * fine;
+    // permutation, corners and folded values (one point of each opposite pair),
+    // the covered half of the fine grid; not below the footprint of the whole grid
+    b += std::max(4 * M + 3 * 8 * fine, 7 * (M + nt) + 14 * fine);
     b += 4 * nv * vecs;
     b += 4 * (size_t)j.recon_dims[0] * j.recon_dims[1] * j.recon_dims[2];
     b += Toeplitz::work_bytes(N, true) + Toeplitz::build_peak_bytes(N, true);

@@ -49,3 +49,40 @@ def test_3d(cuda, rows, cols, shifted):
     x = rng.standard_normal(dims).astype(np.float32)
     assert O.rel_l2(lc.forward(x, pg).cpu().numpy(), O.forward3d(x, g)) < 1e-5
     assert O.rel_l2(lc.sysmat(x, pg).cpu().numpy(), O.sysmat3d_nufft(x.astype(np.float64), g)) < 1e-5
+
+
+# Angles whose lattices coincide share one set of points: theta and theta + 180
+# degrees (opposite radii in 2D, mirrored rows in 3D without a second tilt) and
+# repeated angles, in any order, each with its own shift.  Angle counts leave
+# representatives with one, two and three members.
+@pytest.mark.parametrize("n", [12, 17])
+def test_2d_coinciding_angles(cuda, n):
+    import laminocam_b200 as lc
+    rng = np.random.default_rng(n)
+    t = rng.uniform(-3, 3, 4)
+    theta = np.concatenate([t, [t[0]], t[:3] + np.pi, [t[1] - np.pi]])
+    pg = lc.PolarGrid2D(theta, n)
+    y = rng.standard_normal((2, len(theta), n)).astype(np.float32)
+    assert O.rel_l2(lc.backproj2d(y, pg, (2, n, n)).cpu().numpy(), O.backproj2d(y, theta, (2, n, n))) < 1e-5
+    x = rng.standard_normal((2, n, n)).astype(np.float32)
+    assert O.rel_l2(lc.forward2d(x, pg).cpu().numpy(), O.forward2d(x, theta, n)) < 1e-5
+
+
+@pytest.mark.parametrize("rows,cols", [(8, 9), (9, 8), (9, 11), (8, 8), (57, 61)])
+@pytest.mark.parametrize("shifted", [False, True])
+@pytest.mark.parametrize("beta", [0.0, 0.2])
+def test_3d_coinciding_angles(cuda, rows, cols, shifted, beta):
+    import laminocam_b200 as lc
+    rng = np.random.default_rng(rows * 100 + cols)
+    dims = (5, 9, 8)
+    t = np.array([0.0, 0.7, np.pi / 2])
+    theta = np.concatenate([t, t[::-1] + np.pi, [0.7], [2.9]])
+    nth = len(theta)
+    gamma, bt = np.full(nth, -0.61), np.full(nth, beta)
+    sh = rng.uniform(-2, 2, (nth, 2)).astype(np.float32) if shifted else None
+    pg = lc.PolarGrid(theta, gamma, bt, rows, cols, sh)
+    g = O.Grid3D(theta, gamma, bt, rows, cols)
+    y = rng.standard_normal((nth, rows, cols)).astype(np.float32)
+    assert O.rel_l2(lc.backproj(y, pg, dims, shifts=shifted).cpu().numpy(), O.backproj3d(y, g, dims, sh)) < 1e-5
+    x = rng.standard_normal(dims).astype(np.float32)
+    assert O.rel_l2(lc.forward(x, pg).cpu().numpy(), O.forward3d(x, g)) < 1e-5
