@@ -700,7 +700,9 @@ void launch_axis_fft(Context &ctx, const AxisFFT &a) {
     else if (a.out_map == OUT_REAL_UNPACK) LC_REQUIRE(a.n_out <= 2 * a.L, "axis FFT: n_out > 2L");
     else LC_REQUIRE(a.n_out <= a.L, "axis FFT: n_out > L");
     if (a.n_outer <= 0 || a.n_inner <= 0 || a.n_out == 0) return;
-    if (line_kernels_enabled() && (launch_col_fft(ctx.stream(), a) || launch_row_fft(ctx.stream(), a))) return;
+    if (line_kernels_enabled() &&
+        (launch_col_fft(ctx.stream(), a) || launch_row_fft(ctx.stream(), a) || launch_mode_fft(ctx.stream(), a)))
+        return;
     LC_REQUIRE(a.cg_parts == 0, "axis FFT: fused CG work needs a register-plan row kernel");
 
     const FFTPlan &pl = ctx.plans().get(a.L, a.fp64, ctx.stream());

@@ -176,6 +176,11 @@ bool launch_col_fft(cudaStream_t st, const AxisFFT &a);
 // Returns false otherwise.  launch_axis_fft tries it first.
 bool launch_row_fft(cudaStream_t st, const AxisFFT &a);
 
+// NUFFT passes between an even fine-grid length and modes that fill at most half
+// of it (IN_MODES, OUT_MODES; the grid side whole or as a window), on the
+// register plans.  Returns false otherwise.  launch_axis_fft tries it first.
+bool launch_mode_fft(cudaStream_t st, const AxisFFT &a);
+
 // false when LC_LINE_KERNELS=0: every transform then takes the generic
 // shared-memory kernel (A/B timing of the register-plan kernels)
 bool line_kernels_enabled();
