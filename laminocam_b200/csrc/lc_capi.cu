@@ -55,26 +55,30 @@ __global__ void max_kernel(const float *__restrict__ a, long n, unsigned *out_bi
     }
 }
 
-// out {nt, N2, N3} = in {nt, n2, n3} / scale placed at (d2, d3), zero elsewhere
-__global__ void norm_pad_kernel(const float *__restrict__ in, long nt, long n2, long n3,
-                                float *__restrict__ out, long N2, long N3, long d2, long d3,
-                                const unsigned *max_bits) {
+// out {nt, N2, N3} = in {nt, n2, n3} / scale placed at (d2, d3), zero elsewhere;
+// one block per output row (the division of a linear index per value took
+// 0.66 ms for 360 x 721 x 721 values, 1.1 GB of traffic)
+__global__ void __launch_bounds__(256) norm_pad_kernel(const float *__restrict__ in, int n2, int n3,
+                                                       float *__restrict__ out, long rows, int N2, int N3, int d2,
+                                                       int d3, const unsigned *max_bits) {
     unsigned b = *max_bits;
     b = (b & 0x80000000u) ? (b & 0x7fffffffu) : ~b;
-    float mx = __uint_as_float(b);
-    bool scale = mx > 0.f;
-    long total = nt * N2 * N3;
-    for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (long)gridDim.x * blockDim.x) {
-        long t = idx / (N2 * N3);
-        long r = idx - t * N2 * N3;
-        long j = r / N3 - d2, k = r % N3 - d3;
-        float v = 0.f;
-        if (j >= 0 && j < n2 && k >= 0 && k < n3) {
-            v = in[(t * n2 + j) * n3 + k];
-            if (scale) v = v / mx;
+    const float mx = __uint_as_float(b);
+    const bool scale = mx > 0.f;
+    for (long row = blockIdx.x; row < rows; row += gridDim.x) {
+        const long t = row / N2;
+        const int j = (int)(row - t * N2) - d2;
+        const bool in_row = j >= 0 && j < n2;
+        const float *src = in + (t * n2 + j) * (long)n3;
+        for (int c = threadIdx.x; c < N3; c += blockDim.x) {
+            const int k = c - d3;
+            float v = 0.f;
+            if (in_row && k >= 0 && k < n3) {
+                v = src[k];
+                if (scale) v = v / mx;
+            }
+            out[row * N3 + c] = v;
         }
-        out[idx] = v;
     }
 }
 
@@ -800,9 +804,10 @@ void mbir3d_core(lc_context c, const float *dprojs_in, int ntheta, int nrows, in
     max_kernel<<<grid_for(np, 256, ctx.num_sms()), 256, 0, s>>>(dprojs_in, np, mx.get());
     LC_CHECK_LAUNCH();
     DevBuf<float> dproj((long)ntheta * PR * PC, s);
-    norm_pad_kernel<<<grid_for((long)ntheta * PR * PC, 256, ctx.num_sms()), 256, 0, s>>>(
-        dprojs_in, ntheta, nrows, ncols, dproj.get(), PR, PC, (PR - nrows) / 2, (PC - ncols) / 2,
-        mx.get());
+    const long prows = (long)ntheta * PR;
+    norm_pad_kernel<<<(unsigned)std::min<long>(prows, (long)ctx.num_sms() * 64), 256, 0, s>>>(
+        dprojs_in, nrows, ncols, dproj.get(), prows, (int)PR, (int)PC, (int)((PR - nrows) / 2),
+        (int)((PC - ncols) / 2), mx.get());
     LC_CHECK_LAUNCH();
     const long nvp = N[0] * N[1] * N[2];
     DevBuf<float> yT(nvp, s), x(nvp, s);
