@@ -953,7 +953,10 @@ def main():
         sms = torch.cuda.get_device_properties(local).multi_processor_count
         mhz = clk.summary().get("sm_mhz") or 1965.0
         w = 7  # ES kernel width at NUFFT tolerance 1e-6
-        cells = float(NANGLES) * PADDED_DET[0] * PADDED_DET[1] * w ** 3
+        # one point stands for each pair of opposite lattice points, and over a
+        # full turn of an even number of angles for both angles of a pair
+        pts = ((PADDED_DET[0] * PADDED_DET[1] + 1) // 2) * (NANGLES // 2 if NANGLES % 2 == 0 else NANGLES)
+        cells = float(pts) * w ** 3
         bound_ms = cells * 2.0 / (SHARED_RED_PER_CLK_SM * sms * mhz * 1e6) * 1e3
         spread_roof = {"bound": "shared-memory reductions", "cell_updates": cells,
                        "reductions_per_cell": 2, "peak_reductions_per_clk_per_sm": SHARED_RED_PER_CLK_SM,
