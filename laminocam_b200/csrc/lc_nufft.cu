@@ -409,6 +409,10 @@ __device__ __forceinline__ float2 direct_value(const PolarPts &p, const float2 *
 // Type 2 of a real volume has C(-x) = conj C(x): the value at a folded point
 // goes to both lattice points of the pair, in every member angle (zero outside
 // the band; only lattice points below keep are stored).
+// keep < lat: the caller takes the values as Hermitian, for the real part of
+// their transform.  That part keeps the mean of a value and its opposite's
+// conjugate.  On the band limit rounding can put one of them in and the other
+// out, so both get the mean of the pair's two flags.
 __global__ void __launch_bounds__(256) expand_values_kernel(PolarPts pts, const float2 *__restrict__ vals, int nvol,
                                                             int mode, int keep, float2 *__restrict__ c) {
     const bool band = mode != PT_PLAIN && pts.dim == 3;
@@ -422,12 +426,14 @@ __global__ void __launch_bounds__(256) expand_values_kernel(PolarPts pts, const 
             const int l = member_point(pts, pi.l, mb.y), o = pts.lat - 1 - l;
             const bool st_l = l < keep, st_o = o != l && o < keep;
             const bool in_l = !band || point_in_band(pts, mb.x, l), in_o = !band || point_in_band(pts, mb.x, o);
+            const bool split = keep < pts.lat && in_l != in_o;
             float2 *a = c + (long)mb.x * pts.lat;
             for (int s = 0; s < nvol; ++s) {
                 float2 v = vals[(long)s * pts.Mh + j];
                 if (pi.flip) v.y = -v.y;
-                if (st_l) a[(long)s * pts.M + l] = in_l ? v : zero;
-                if (st_o) a[(long)s * pts.M + o] = in_o ? cconj(v) : zero;
+                if (split) v = cscale(v, 0.5f);
+                if (st_l) a[(long)s * pts.M + l] = in_l || split ? v : zero;
+                if (st_o) a[(long)s * pts.M + o] = in_o || split ? cconj(v) : zero;
             }
         }
     }

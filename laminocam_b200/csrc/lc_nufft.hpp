@@ -102,7 +102,8 @@ class NufftPlan {
     void type1_real(Context &ctx, const float2 *c, int nvol, float *out, float scale,
                     PtMode mode, bool herm = false);
     // type 2: real in [nvol][...modes] -> c [nvol][M].  keep > 0: only lattice
-    // points below it (and at least half) are stored.
+    // points below it (and at least half) are stored, and the caller takes the
+    // others as their conjugates (see expand_values_kernel for the band limit).
     void type2_real(Context &ctx, const float *in, int nvol, float2 *c, PtMode mode, int keep = 0);
 
     int dim() const { return dim_; }
