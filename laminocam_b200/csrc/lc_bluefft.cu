@@ -42,6 +42,7 @@ struct BlueArgs {
     void *out;
     long n_outer, n_inner, in_ostride, out_ostride, bpo;
     long rows_per, group_stride;
+    long lines, lines_per;  // rows: complex lines in all and per group
     int n, d_pre, d_post, out_min, out_max, herm;
     float scale;
     const float2 *chirp, *V;
@@ -83,14 +84,15 @@ __global__ void __launch_bounds__(RegPlan<R0, R1, R2>::NT *kBlueLines) blue_kern
     bool valid, valid_b = false;
     int col = 0;  // column of a C2C column line
     if constexpr (ROWS) {
-        const long l0 = ((long)blockIdx.x * C + c) * (PAIR ? 2 : 1);
-        valid = l0 < a.n_outer;
-        valid_b = PAIR && l0 + 1 < a.n_outer;
+        constexpr int K = PAIR ? 2 : 1;  // rows of a line
+        const long l0 = (long)blockIdx.x * C + c;
+        valid = l0 < a.lines;
         const long line = valid ? l0 : 0;
-        const long g = line / a.rows_per, r = line - g * a.rows_per;
+        const long g = line / a.lines_per, r = K * (line - g * a.lines_per);
+        valid_b = PAIR && valid && r + 1 < a.rows_per;
         base_in = g * a.group_stride + r * a.in_ostride;
         base_out = g * a.group_stride + r * a.out_ostride;
-        if constexpr (PAIR) {  // pairs run over ungrouped rows
+        if constexpr (PAIR) {
             sec_in = a.in_ostride;
             sec_out = a.out_ostride;
         }
@@ -273,7 +275,7 @@ bool launch_bluestein_lines(cudaStream_t st, const AxisDFT &a, const BluesteinEn
     if (a.n_outer <= 0 || a.n_inner <= 0) return true;
     const int kind = rows ? (in_real ? BK_ROWS_R2C : (out_real ? BK_ROWS_C2R : BK_ROWS_C2C))
                           : (out_real ? BK_COLS_C2R : BK_COLS_C2C);
-    LC_REQUIRE(a.rows_per == 0 || kind == BK_ROWS_C2C, "DFT: only complex rows come in groups");
+    LC_REQUIRE(a.rows_per == 0 || (rows && a.n_outer % a.rows_per == 0), "DFT: rows come in whole groups");
     LC_REQUIRE((a.out_min == 0 && a.out_max == 0) || kind == BK_ROWS_R2C, "DFT: only real rows are stored in part");
     LC_REQUIRE(!a.herm || (!rows && a.n % 2 == 1 && (out_real || a.n_inner % 2 == 1)),
                "DFT: Hermitian columns need odd sizes");
@@ -299,8 +301,9 @@ bool launch_bluestein_lines(cudaStream_t st, const AxisDFT &a, const BluesteinEn
     const bool pair = kind == BK_ROWS_R2C || kind == BK_ROWS_C2R || kind == BK_COLS_C2R;
     long blocks;
     if (rows) {
-        const long lines = pair ? (a.n_outer + 1) / 2 : a.n_outer;
-        blocks = (lines + kBlueLines - 1) / kBlueLines;
+        b.lines_per = pair ? (b.rows_per + 1) / 2 : b.rows_per;
+        b.lines = a.n_outer / b.rows_per * b.lines_per;
+        blocks = (b.lines + kBlueLines - 1) / kBlueLines;
         b.bpo = 1;
     } else {
         const long cols = pair ? (a.n_inner + 1) / 2 : (a.herm ? a.n_inner - a.n_inner / 2 : a.n_inner);

@@ -100,6 +100,23 @@ void launch_chained(void (*kern)(P...), unsigned grid, unsigned block, size_t sm
     LC_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
 }
 
+// n / d for 0 <= n < 2^31 by a multiply and a shift (Granlund and Montgomery,
+// "Division by invariant integers using multiplication", PLDI 1994): with
+// 2^(s-1) < d <= 2^s and m = floor(2^32 (2^s - d) / d) + 1,
+// n / d = (umulhi(n, m) + n) >> s  (the sum stays below 2^32 for n < 2^31).
+struct FastDiv {
+    unsigned m = 1, s = 0;
+};
+
+inline FastDiv make_fastdiv(unsigned d) {
+    FastDiv f;
+    while ((1ull << f.s) < d) ++f.s;
+    f.m = (unsigned)(((1ull << 32) * ((1ull << f.s) - d)) / d + 1);
+    return f;
+}
+
+__device__ __forceinline__ unsigned fast_div(unsigned n, FastDiv f) { return (__umulhi(n, f.m) + n) >> f.s; }
+
 // ---------------------------------------------------------------------------
 // complex arithmetic
 // ---------------------------------------------------------------------------

@@ -55,6 +55,10 @@ struct AxisFFT {
     OutMap out_map = OUT_DIRECT;
     int out_off = 0;
     int in_shift = -1, out_shift = -1;
+    // rows (n_inner == 1) of one independent problem (0: all): real rows that
+    // share a complex line are taken from the same one, so that neither rounding
+    // errors nor NaN reach from one problem into the next
+    long problem_rows = 0;
     int sign = -1;
     const void *pre = nullptr;      // real factor per input index j
     const void *linefac = nullptr;  // real factor per line inner index c
@@ -205,7 +209,10 @@ struct AxisDFT {
     // Lines of data that is Hermitian about a stored centre; only lengths with
     // dft_on_lines(n) take these.
     // Rows (n_inner == 1) in groups: line g * rows_per + r is at
-    // g * group_stride + r * stride (0: the lines follow one another).
+    // g * group_stride + r * stride (0: the lines follow one another).  Two
+    // real lines share a complex one only within a group: the slices of a stack
+    // are independent problems, and rounding errors or NaN of one stay out of
+    // the next.
     long rows_per = 0, group_stride = 0;
     // Real rows: store only the outputs k in [out_min, out_max) (out_max 0: n).
     int out_min = 0, out_max = 0;

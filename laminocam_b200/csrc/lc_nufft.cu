@@ -248,8 +248,6 @@ struct GridCfg {
     float beta_l2e;          // ES beta times log2(e)
 };
 
-__device__ __forceinline__ unsigned fast_div(unsigned n, FastDiv f) { return (__umulhi(n, f.m) + n) >> f.s; }
-
 struct PointInfo {
     double c[3];  // x, y, z
     double qX, qY;

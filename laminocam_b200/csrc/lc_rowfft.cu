@@ -15,7 +15,7 @@
 // transform, and once more in the forward unpack (which pairs k with M - k).
 //
 // Real lines of odd length M (81, 243, 729: the next 2^p 3^q of some sizes is a
-// power of three) go two to a complex line, z = a + i b:
+// power of three) go two rows of one slice or volume to a complex line, z = a + i b:
 //   forward  A[k] = (Z[k] + conj Z[M-k]) / 2,  B[k] = (Z[k] - conj Z[M-k]) / 2i
 //   inverse  Z[k] = A[k] + i B[k],  Z[M-k] = conj A[k] + i conj B[k]
 // (11160 rows of 729 points: the generic kernel, one complex line per row, took
@@ -42,6 +42,10 @@ struct RowArgs {
     const void *in;
     void *out;
     long n_lines, in_stride, out_stride;
+    // odd lengths: rows of one problem (pairs stay within it), whether odd, and
+    // the division of a pair's number by the pairs of a problem
+    int problem_rows, odd_rows;
+    FastDiv div_pairs;
     int n_in, n_out;
     float scale;
     // fused CG work (R2C: direction update of the input; C2R: p . output)
@@ -66,14 +70,21 @@ __device__ __forceinline__ void row_fft_body(const RowArgs &a, long bid) {
     load_line_twiddles<M>(tw);
     chain_wait();
     const int t = threadIdx.x % NT, c = threadIdx.x / NT;
-    const long line = (bid * kRowLines + c) * row_reals(MODE);  // odd lengths: and line + 1
+    long line = bid * kRowLines + c;
+    bool pair = false;  // odd lengths: line + 1 as well
+    if constexpr (row_reals(MODE) == 2) {
+        // pair number -> problem (g) and first row
+        const unsigned p = (unsigned)line, g = fast_div(p, a.div_pairs);
+        line = 2 * (long)p - (a.odd_rows ? g : 0u);
+        pair = line + 1 < (long)(g + 1) * a.problem_rows;
+    }
     const bool valid = line < a.n_lines;
     float2 *buf = row_sm + c * M;
     const auto at = [&](int, int i) -> float2 & { return buf[i]; };
     constexpr int NA = M / R0;
     float2 v[1][RM];
     if constexpr (MODE == RM_ODD_R2C || MODE == RM_ODD_C2R) {
-        const bool valid_b = line + 1 < a.n_lines;
+        const bool valid_b = valid && pair;
         const long li = (valid ? line : 0) * a.in_stride, lo = (valid ? line : 0) * a.out_stride;
         const float2 zero = make_float2(0.f, 0.f);
         if (t < NA) {
@@ -390,8 +401,17 @@ bool launch_row_fft(cudaStream_t st, const AxisFFT &a) {
         ra.cg_upd = (mode == RM_R2C && (a.cg_parts & kFusedUpdate)) ? 1 : 0;
         ra.cg_dot = (mode == RM_C2R && (a.cg_parts & kFusedDot)) ? 1 : 0;
     }
-    const int reals = row_reals(mode);
-    const long blocks = row_fft_ctas((a.n_outer + reals - 1) / reals);
+    long lines = a.n_outer;
+    if (row_reals(mode) == 2) {
+        const long rows = a.problem_rows > 0 ? a.problem_rows : a.n_outer, pairs = (rows + 1) / 2;
+        LC_REQUIRE(a.n_outer % rows == 0, "row FFT: problems of unequal size");
+        lines = a.n_outer / rows * pairs;
+        LC_REQUIRE(lines + kRowLines < (1L << 31), "row FFT: too many rows");
+        ra.problem_rows = (int)rows;
+        ra.odd_rows = (int)(rows % 2);
+        ra.div_pairs = make_fastdiv((unsigned)pairs);
+    }
+    const long blocks = row_fft_ctas(lines);
     LC_REQUIRE(blocks < (1L << 31), "row FFT: grid too large");
     return launch_row_plan(st, M, mode, ra, blocks);
 }

@@ -1234,6 +1234,7 @@ void Toeplitz::apply(Context &ctx, const float *x, float *y, const CGFusion *f, 
         a.out_t = E_C64;
         a.n_outer = n1 * n2;
         a.n_inner = 1;
+        if (!three_d_) a.problem_rows = n2;  // a slice
         a.in_ostride = pitch;
         a.out_ostride = P3h;
         a.n_in = (int)n3;
@@ -1346,6 +1347,7 @@ void Toeplitz::apply(Context &ctx, const float *x, float *y, const CGFusion *f, 
         a.out_t = E_F32;
         a.n_outer = n1 * n2;
         a.n_inner = 1;
+        if (!three_d_) a.problem_rows = n2;  // a slice
         a.in_ostride = P3h;
         a.out_ostride = pitch;
         a.n_in = P3h;
