@@ -628,12 +628,16 @@ constexpr unsigned kRoundMagicBits = 0x4B400000u;
 // bound on the sum of the weights of the bin's footprints over one cell.  W_b
 // exceeds the largest sum by its margins of 1e-3 per axis and 1e-4, above
 // 2^20 steps of a sum near 2^31, so the sum and its at most 1024 rounding
-// halves stay below 2^31; and e_b <= e_G.
+// halves stay below 2^31; and e_b <= e_G.  e_G <= 126 keeps both scales finite
+// floats for values down to the smallest (the step is then the smallest normal
+// float, 2^-126).
+constexpr int kMaxFixExponent = 126;
+
 __host__ __device__ __forceinline__ int fix_exponent_grid(float m, long kmax) {
     if (!(m > 0.f)) return 0;
     int e3;
     frexp((double)kmax * (double)m, &e3);  // kmax m < 2^e3
-    return 61 - e3;
+    return 61 - e3 < kMaxFixExponent ? 61 - e3 : kMaxFixExponent;
 }
 
 __device__ __forceinline__ int fix_exponent_tile(float mb, float wb, int eg) {
