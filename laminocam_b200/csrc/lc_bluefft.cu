@@ -42,7 +42,8 @@ struct BlueArgs {
     void *out;
     long n_outer, n_inner, in_ostride, out_ostride, bpo;
     long rows_per, group_stride;
-    long lines, lines_per;  // rows: complex lines in all and per group
+    int odd_rows;       // pairs: whether a group has an odd number of rows, and the
+    FastDiv div_lines;  // division of a line's number by the lines of a group
     int n, d_pre, d_post, out_min, out_max, herm;
     float scale;
     const float2 *chirp, *V;
@@ -84,17 +85,22 @@ __global__ void __launch_bounds__(RegPlan<R0, R1, R2>::NT *kBlueLines) blue_kern
     bool valid, valid_b = false;
     int col = 0;  // column of a C2C column line
     if constexpr (ROWS) {
-        constexpr int K = PAIR ? 2 : 1;  // rows of a line
-        const long l0 = (long)blockIdx.x * C + c;
-        valid = l0 < a.lines;
-        const long line = valid ? l0 : 0;
-        const long g = line / a.lines_per, r = K * (line - g * a.lines_per);
-        valid_b = PAIR && valid && r + 1 < a.rows_per;
-        base_in = g * a.group_stride + r * a.in_ostride;
-        base_out = g * a.group_stride + r * a.out_ostride;
         if constexpr (PAIR) {
+            const unsigned line = blockIdx.x * C + c, g = fast_div(line, a.div_lines);
+            const long l0 = 2 * (long)line - (a.odd_rows ? g : 0u);
+            valid = l0 < a.n_outer;
+            valid_b = l0 + 1 < (long)(g + 1) * a.rows_per && valid;
+            base_in = (valid ? l0 : 0) * a.in_ostride;
+            base_out = (valid ? l0 : 0) * a.out_ostride;
             sec_in = a.in_ostride;
             sec_out = a.out_ostride;
+        } else {
+            const long l0 = (long)blockIdx.x * C + c;
+            valid = l0 < a.n_outer;
+            const long line = valid ? l0 : 0;
+            const long g = line / a.rows_per, r = line - g * a.rows_per;
+            base_in = g * a.group_stride + r * a.in_ostride;
+            base_out = g * a.group_stride + r * a.out_ostride;
         }
         step = 1;
     } else {
@@ -275,7 +281,9 @@ bool launch_bluestein_lines(cudaStream_t st, const AxisDFT &a, const BluesteinEn
     if (a.n_outer <= 0 || a.n_inner <= 0) return true;
     const int kind = rows ? (in_real ? BK_ROWS_R2C : (out_real ? BK_ROWS_C2R : BK_ROWS_C2C))
                           : (out_real ? BK_COLS_C2R : BK_COLS_C2C);
+    const bool pair = kind == BK_ROWS_R2C || kind == BK_ROWS_C2R || kind == BK_COLS_C2R;
     LC_REQUIRE(a.rows_per == 0 || (rows && a.n_outer % a.rows_per == 0), "DFT: rows come in whole groups");
+    LC_REQUIRE(a.group_stride == 0 || (a.rows_per > 0 && !pair), "DFT: real lines follow one another");
     LC_REQUIRE((a.out_min == 0 && a.out_max == 0) || kind == BK_ROWS_R2C, "DFT: only real rows are stored in part");
     LC_REQUIRE(!a.herm || (!rows && a.n % 2 == 1 && (out_real || a.n_inner % 2 == 1)),
                "DFT: Hermitian columns need odd sizes");
@@ -298,12 +306,13 @@ bool launch_bluestein_lines(cudaStream_t st, const AxisDFT &a, const BluesteinEn
     b.scale = a.scale;
     b.chirp = e.chirp.get();
     b.V = e.V.get();
-    const bool pair = kind == BK_ROWS_R2C || kind == BK_ROWS_C2R || kind == BK_COLS_C2R;
     long blocks;
     if (rows) {
-        b.lines_per = pair ? (b.rows_per + 1) / 2 : b.rows_per;
-        b.lines = a.n_outer / b.rows_per * b.lines_per;
-        blocks = (b.lines + kBlueLines - 1) / kBlueLines;
+        const long lines_per = pair ? (b.rows_per + 1) / 2 : b.rows_per, lines = a.n_outer / b.rows_per * lines_per;
+        LC_REQUIRE(lines + kBlueLines < (1L << 31), "DFT: too many lines");
+        b.odd_rows = (int)(b.rows_per % 2);
+        b.div_lines = make_fastdiv((unsigned)lines_per);
+        blocks = (lines + kBlueLines - 1) / kBlueLines;
         b.bpo = 1;
     } else {
         const long cols = pair ? (a.n_inner + 1) / 2 : (a.herm ? a.n_inner - a.n_inner / 2 : a.n_inner);

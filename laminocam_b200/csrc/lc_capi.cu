@@ -148,10 +148,7 @@ void do_forward2d(lc_geometry g, const float *vol, int ns, int n2, int n3, float
     d.d_post = nr / 2;       // fftshift1
     d.sign = +1;
     d.scale = 1.0f / (float)nr;
-    if (dft_on_lines(nr)) {  // a slice's angles
-        d.rows_per = nth;
-        d.group_stride = (long)nth * nr;
-    }
+    if (dft_on_lines(nr)) d.rows_per = nth;  // of a slice
     launch_axis_dft(ctx, d);
 }
 

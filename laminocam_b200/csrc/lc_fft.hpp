@@ -208,11 +208,11 @@ struct AxisDFT {
     float scale = 1.0f;
     // Lines of data that is Hermitian about a stored centre; only lengths with
     // dft_on_lines(n) take these.
-    // Rows (n_inner == 1) in groups: line g * rows_per + r is at
-    // g * group_stride + r * stride (0: the lines follow one another).  Two
-    // real lines share a complex one only within a group: the slices of a stack
-    // are independent problems, and rounding errors or NaN of one stay out of
-    // the next.
+    // Rows (n_inner == 1) in groups of rows_per.  Complex lines: line
+    // g * rows_per + r is at g * group_stride + r * stride.  Lines that are real
+    // on one side follow one another, and two of them share a complex one only
+    // within a group: the slices of a stack are independent problems, and
+    // rounding errors or NaN of one stay out of the next.
     long rows_per = 0, group_stride = 0;
     // Real rows: store only the outputs k in [out_min, out_max) (out_max 0: n).
     int out_min = 0, out_max = 0;
