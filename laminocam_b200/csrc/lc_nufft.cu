@@ -51,6 +51,28 @@ static void set_lattice(Context &ctx, PolarGeometry &g, int lat, const std::vect
         const std::array<int, 2> &s0 = sign0[it->second];
         reps[it->second].push_back(make_int2(i, (sg[0] != s0[0] ? 1 : 0) | (sg[1] != s0[1] ? 2 : 0)));
     }
+    // 2D: the fold and expand passes are two more passes over the values, which
+    // the spreading and the interpolation otherwise read and write themselves
+    // (Direct2D), so sharing pays only where it saves many angles.  Shared
+    // against direct, us per backprojection (projection):
+    //   511^2, 360 angles, one coinciding      78.6 (52.7)   74.5 (46.8)
+    //   1023^2, 720 angles, one coinciding    150.6 (111.1) 140.8 (102.2)
+    //   1535^2, 1080 angles, third saved      305.9 (232.1) 305.9 (228.2)
+    //   1535^2, 1080 angles, 41 % saved       296.5 (227.8) 301.6 (225.5)
+    //   2047^2, 1440 angles, quarter saved    536.6 (398.3) 536.8 (388.5)
+    //   2047^2, 1440 angles, third saved      517.3 (387.3) 527.1 (383.2)
+    //   2047^2, 1440 angles, 41 % saved       502.6 (376.8) 514.4 (378.0)
+    //   2047^2, full turn (half saved)        483.2 (365.3) 504.8 (372.4)
+    //   1023^2, full turn                     128.6 (98.4)  127.7 (96.2)
+    //   511^2, full turn                       74.9 (53.4)   71.9 (47.3)
+    // The line is at two fifths of the angles.  Small full turns stay shared
+    // although they are slower so: values that coincide are added as floats
+    // instead of each being rounded to the bin's step, and the sums are closer to
+    // 64 bits (4000 angles on 96^2, noise: 3.0e-6 shared, 6.9e-6 direct).
+    if (p.dim == 2 && 5L * (p.ntheta - (long)reps.size()) < 2L * p.ntheta) {
+        reps.clear();
+        for (int i = 0; i < p.ntheta; ++i) reps.push_back({make_int2(i, 0)});
+    }
     std::vector<int> off{0};
     std::vector<int2> mem;
     for (const auto &r : reps) {
@@ -379,10 +401,8 @@ __global__ void __launch_bounds__(256) fold_values_kernel(PolarPts pts, const fl
     }
 }
 
-// In 2D, where no two angles share a lattice, the spreading and the
-// interpolation read and write the lattice values themselves: the two passes
-// would cost more than they save (four 511^2 slices: projection 103 -> 108 us,
-// four 1023^2 slices: backprojection 439 -> 453 us with them).
+// In 2D, where every angle is its own representative (set_lattice), the
+// spreading and the interpolation read and write the lattice values themselves.
 struct Direct2D {
     int on;    // the values are the lattice's, [nvol][M], not folded ones
     int herm;  // type 1: opposite values are conjugates, only l < half is stored

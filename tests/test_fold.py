@@ -68,6 +68,23 @@ def test_2d_coinciding_angles(cuda, n):
     assert O.rel_l2(lc.forward2d(x, pg).cpu().numpy(), O.forward2d(x, theta, n)) < 1e-5
 
 
+# 2D angles share points only where that saves two fifths of them: either side
+# of the line, one coinciding pair, a full turn, both parities, and more slices
+# than one chunk of the shared-memory tiles holds (eight).
+@pytest.mark.parametrize("nth,saved", [(41, 1), (41, 16), (41, 17), (40, 20)])
+@pytest.mark.parametrize("n,ns", [(20, 1), (21, 9), (20, 17)])
+def test_2d_share_of_coinciding_angles(cuda, nth, saved, n, ns):
+    import laminocam_b200 as lc
+    rng = np.random.default_rng(100 * nth + saved + n)
+    theta = rng.permutation(np.linspace(0.0, np.pi, nth - saved, endpoint=False))
+    theta = np.concatenate([theta, theta[:saved] + np.pi * rng.integers(-1, 2, saved)])
+    pg = lc.PolarGrid2D(theta, n)
+    y = rng.standard_normal((ns, nth, n)).astype(np.float32)
+    x = rng.standard_normal((ns, n, n)).astype(np.float32)
+    assert O.rel_l2(lc.backproj2d(y, pg, (ns, n, n)).cpu().numpy(), O.backproj2d(y, theta, (ns, n, n))) < 1e-5
+    assert O.rel_l2(lc.forward2d(x, pg).cpu().numpy(), O.forward2d(x, theta, n)) < 1e-5
+
+
 @pytest.mark.parametrize("rows,cols", [(8, 9), (9, 8), (9, 11), (8, 8), (57, 61)])
 @pytest.mark.parametrize("shifted", [False, True])
 @pytest.mark.parametrize("beta", [0.0, 0.2])
