@@ -1342,6 +1342,58 @@ GridCfg make_cfg(int dim, const int nf[3], const int bs[3], const int nb[3], int
 // ---------------------------------------------------------------------------
 // plan
 // ---------------------------------------------------------------------------
+// Fine-grid lengths and the kept rows (ny from row -ylo) of a plan.
+static void plan_sizes(int dim, const long modes[3], int w, long nf[3], int &ylo, long &ny) {
+    for (int d = 0; d < 3; ++d) {
+        // The next 2^p 3^q; where that is a power of three (243, 729, 2187) the
+        // next even one, 5 % longer, whose passes run on the register plans
+        // (projection 180 x 361 x 361, 729 -> 768 cells: 1503 -> 1465 us; below
+        // 128 cells there is no plan and the odd length stays).
+        long n = next_smooth23(std::max(2 * modes[d], 2L * w));
+        if (n % 2 != 0) {
+            long e = n;
+            while (e % 2 != 0) e = next_smooth23(e + 1);
+            if (e < 8192 && line_plan_exists((int)(e / 2))) n = e;
+        }
+        nf[d] = d < dim ? n : 1;
+    }
+    // Folded points have u = y nf / 2 pi in [0, nf / 2] up to rounding, so
+    // footprints cover the rows -w/2 - 1 .. nf/2 + w/2 + 2 at most.  Only those
+    // are stored, cleared, converted and transformed along x; the y pass takes
+    // (type 1) or leaves (type 2) them as a window.  (Backprojection of four
+    // 1023^2 slices, 4 x 2048^2 cells: 0.59 -> 0.44 ms.)
+    ylo = w / 2 + 1;
+    ny = nf[1] / 2 + 2 * (w / 2) + 4;
+    if (ny >= nf[1]) {
+        ylo = 0;
+        ny = nf[1];
+    }
+}
+
+constexpr int kBins2[3] = {32, 32, 1}, kBins3[3] = {16, 8, 8};  // cells of a bin
+
+size_t NufftPlan::device_bytes(int dim, const long modes[3], double tol, long ntheta, long lat, long nvol) {
+    const int w = es_width_for_tol(tol);
+    long nf[3], ny;
+    int ylo;
+    plan_sizes(dim, modes, w, nf, ylo, ny);
+    const size_t n1 = dim == 3 ? modes[2] : 1, n2 = modes[1], n3 = modes[0];
+    // every angle as its own representative: permutation, corner, folded values
+    const size_t pts = (size_t)ntheta * ((lat + 1) / 2);
+    size_t b = pts * (sizeof(int) + sizeof(unsigned short) + (size_t)nvol * sizeof(float2));
+    // fine grid, its fixed-point sums, and the passes between it and the modes
+    const size_t rows = (size_t)nf[2] * ny * nvol;
+    b += rows * nf[0] * (sizeof(float2) + 2 * sizeof(long long)) + rows * n3 * sizeof(float2);
+    if (dim == 3) b += (size_t)nvol * nf[2] * n2 * n3 * sizeof(float2) + n2 * n3 * sizeof(float);
+    // deapodisation factors; per bin the counts, positions and bounds (one per
+    // chunk of volumes, at least one volume each), and the subproblems
+    b += (n1 + n2 + n3) * (sizeof(double) + sizeof(float));
+    size_t bins = 1;
+    for (int d = 0; d < dim; ++d) bins *= (nf[d] + (dim == 2 ? kBins2 : kBins3)[d] - 1) / (dim == 2 ? kBins2 : kBins3)[d];
+    b += bins * (5 + nvol) * sizeof(int) + (bins + pts / 1024) * sizeof(int4);
+    return b;
+}
+
 NufftPlan::NufftPlan(Context &ctx, const PolarGeometry &g, const int modes[3], double tol) {
     dim_ = g.pts.dim;
     pts_ = g.pts;
@@ -1351,34 +1403,15 @@ NufftPlan::NufftPlan(Context &ctx, const PolarGeometry &g, const int modes[3], d
     for (int d = 0; d < 3; ++d) {
         modes_[d] = d < dim_ ? modes[d] : 1;
         LC_REQUIRE(modes_[d] >= 1, "NUFFT: mode counts must be positive");
-        // The next 2^p 3^q; where that is a power of three (243, 729, 2187) the
-        // next even one, 5 % longer, whose passes run on the register plans
-        // (projection 180 x 361 x 361, 729 -> 768 cells: 1503 -> 1465 us; below
-        // 128 cells there is no plan and the odd length stays).
-        long nf = next_smooth23(std::max(2 * modes_[d], 2 * w_));
-        if (nf % 2 != 0) {
-            long e = nf;
-            while (e % 2 != 0) e = next_smooth23(e + 1);
-            if (line_plan_exists((int)(e / 2))) nf = e;
-        }
-        nf_[d] = d < dim_ ? (int)nf : 1;
     }
-    // Folded points have u = y nf / 2 pi in [0, nf / 2] up to rounding, so
-    // footprints cover the rows -w/2 - 1 .. nf/2 + w/2 + 2 at most.  Only those
-    // are stored, cleared, converted and transformed along x; the y pass takes
-    // (type 1) or leaves (type 2) them as a window.  (Backprojection of four
-    // 1023^2 slices, 4 x 2048^2 cells: 0.59 -> 0.44 ms.)
-    ylo_ = w_ / 2 + 1;
-    ny_ = nf_[1] / 2 + 2 * (w_ / 2) + 4;
-    if (ny_ >= nf_[1]) {
-        ylo_ = 0;
-        ny_ = nf_[1];
-    }
-    const int bs2[3] = {32, 32, 1};
-    const int bs3[3] = {16, 8, 8};
+    const long lmodes[3] = {modes_[0], modes_[1], modes_[2]};
+    long nf[3], ny;
+    plan_sizes(dim_, lmodes, w_, nf, ylo_, ny);
+    for (int d = 0; d < 3; ++d) nf_[d] = (int)nf[d];
+    ny_ = (int)ny;
     maxsub_ = dim_ == 2 ? 1024 : 2048;
     for (int d = 0; d < 3; ++d) {
-        bs_[d] = std::min(dim_ == 2 ? bs2[d] : bs3[d], nf_[d]);
+        bs_[d] = std::min(dim_ == 2 ? kBins2[d] : kBins3[d], nf_[d]);
         nb_[d] = (nf_[d] + bs_[d] - 1) / bs_[d];
     }
     cudaStream_t st = ctx.stream();

@@ -81,6 +81,9 @@ enum PtMode {
 class NufftPlan {
   public:
     NufftPlan(Context &ctx, const PolarGeometry &g, const int modes[3], double tol);
+    // device memory of a plan over ntheta lattices of lat points and of its
+    // buffers for nvol volumes (an upper bound: angles may share their points)
+    static size_t device_bytes(int dim, const long modes[3], double tol, long ntheta, long lat, long nvol);
     // type 1: c [nvol][M] complex -> out real [nvol][n1][n2][n3] = Re(f) * scale.
     // herm: the values at opposite lattice points are conjugates; only lattice
     // points below half are read.  (Any plan geometry; see fold_values_kernel.)

@@ -177,13 +177,17 @@ size_t next23(long n) { return (size_t)next_smooth23(n); }
 // grids, solver vectors, Toeplitz work buffers and a PSF construction.
 size_t estimate_bytes(const Job &j) {
     const bool sb = j.p.method == 1;
+    const double tol = j.p.nufft_tol > 0 && j.p.nufft_tol < 1 ? j.p.nufft_tol : 1e-6;
     const size_t vecs = 2 + 3 + (sb ? 8 : 0);  // rhs, x; r, p, Ap; d[3], b[3], rhs, x_old
     if (!j.three_d) {
         const size_t ns = j.d0, nt = j.d1, nr = j.d2, n = j.recon_dims[1];
         const size_t M = nt * nr, nv = ns * n * n;
         const size_t nf = next23(std::max<long>(2 * (long)n, 8));
         size_t b = 4 * ns * M + 8 * ns * M;   // sinogram, complex detector lines
-        b += 4 * M + 3 * 8 * nf * nf * ns;     // point permutation, fine grid and pruned passes
+        // NUFFT plan and buffers; not below those of a plan over all points and
+        // the whole fine grid
+        const long modes[3] = {(long)n, (long)n, 1};
+        b += std::max(4 * M + 3 * 8 * nf * nf * ns, NufftPlan::device_bytes(2, modes, tol, nt, nr, ns));
         b += 4 * nv * vecs;
         const long dims[3] = {(long)ns, (long)n, (long)n};
         b += Toeplitz::work_bytes(dims, false) + Toeplitz::build_peak_bytes(dims, false);
@@ -200,9 +204,10 @@ size_t estimate_bytes(const Job &j) {
     const size_t nt = j.d0, M = nt * PR * PC, nv = (size_t)N[0] * N[1] * N[2];
     const size_t fine = next23(2 * N[0]) * next23(2 * N[1]) * next23(2 * N[2]);
     size_t b = 4 * nt * j.d1 * j.d2 + 4 * M + 8 * M;  // raw and padded projections, complex lines
-    // permutation, corners and folded values (one point of each opposite pair),
-    // the covered half of the fine grid; not below the footprint of the whole grid
-    b += std::max(4 * M + 3 * 8 * fine, 7 * (M + nt) + 14 * fine);
+    // NUFFT plan and buffers; not below those of a plan over all points and the
+    // whole fine grid
+    const long modes[3] = {N[2], N[1], N[0]};
+    b += std::max(4 * M + 3 * 8 * fine, NufftPlan::device_bytes(3, modes, tol, nt, PR * PC, 1));
     b += 4 * nv * vecs;
     b += 4 * (size_t)j.recon_dims[0] * j.recon_dims[1] * j.recon_dims[2];
     b += Toeplitz::work_bytes(N, true) + Toeplitz::build_peak_bytes(N, true);
