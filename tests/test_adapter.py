@@ -19,7 +19,8 @@ EXE = os.path.join(ROOT, "oracle", "_ref", "adapter_check")
 
 
 def test_adapter_compiles_against_reference_headers():
-    if not os.path.isdir(os.environ.get("LAMINOCAM_REF", "/root/reference")) and not os.path.exists(EXE):
+    headers = os.path.join(os.environ.get("LAMINOCAM_REF", "/root/reference"), "include", "array.h")
+    if not os.path.exists(headers) and not os.path.exists(EXE):
         pytest.skip("no reference headers to compile against, and no prebuilt check program")
     if not os.path.exists(EXE):
         r = subprocess.run(["make", "-s", "-C", os.path.join(ROOT, "oracle", "ref_build"),
