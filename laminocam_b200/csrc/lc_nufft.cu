@@ -305,10 +305,9 @@ __device__ __forceinline__ void lattice_point(const PolarPts &p, int i, int l, P
 }
 
 // Folded point j: one of each pair of opposite lattice points of a representative
-// angle, negated when
-// its y coordinate (wrapped to [-pi, pi]) is below zero, so that the folded
-// points fill the half of the fine grid with y >= 0 at the density of the
-// full set.
+// angle, negated when its y coordinate (wrapped to [-pi, pi]) is below zero, so
+// that the folded points fill the half of the fine grid with y >= 0 at the
+// density of the full set.
 __device__ __forceinline__ void point_at(const PolarPts &p, long j, PointInfo &pi) {
     const unsigned jj = (unsigned)j;  // below 2^31
     const unsigned r = fast_div(jj, p.div_angle);
@@ -615,8 +614,8 @@ __global__ void bin_scatter_kernel(PolarPts pts, GridCfg g, int W, int *cursor, 
 // which run about four times faster than float atomics in shared memory, one
 // 32-bit word per real and imaginary part of a cell.  Each bin has its own
 // scale F_b = 2^e_b from two bounds over all of its points: m_b, the largest
-// |Re c| + |Im c| of their values (weights are at most 1, and a unit phase
-// keeps each part below |c|), measured per launch, and W_b, a bound on the
+// |Re v| + |Im v| of their folded values (the shifts' phases are in them, and
+// weights are at most 1), measured per launch, and W_b, a bound on the
 // summed kernel weights of the bin's footprints over one tile cell, measured
 // with the plan (the corner histogram of the bin's points, box-summed along
 // each axis with the largest weight each footprint offset can take).
@@ -634,9 +633,11 @@ __global__ void bin_scatter_kernel(PolarPts pts, GridCfg g, int W, int *cursor, 
 // per part of the fine grid, and a conversion pass forms the float grid.
 // Every sum is an exact integer, so the fine grid depends neither on the
 // order of the atomics nor on the schedule: a backprojection is bit-for-bit
-// repeatable.  The rounding step 1 / F_b is at most max(W_b 2^-30, 2^-21) m_b:
-// a cell summed from K footprints is within about sqrt(K / 12) of that of its
-// exact value.
+// repeatable.  The rounding step 1 / F_b is at most the largest of W_b 2^-30 m_b,
+// 2^-21 m_b and, from e_b <= e_G, 2 kmax m 2^-61 (relative to the launch's
+// largest value m: it counts for bins whose values lie far below it), and
+// 2^-126: a cell summed from K footprints is within about sqrt(K / 12) of that
+// of its exact value.
 constexpr int kSpreadThreads = 256;
 constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr unsigned kRoundMagicBits = 0x4B400000u;
@@ -1527,8 +1528,11 @@ void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, Pt
     GridCfg g = make_cfg(dim_, nf_, bs_, nb_, w_, beta_, ylo_, ny_);
     const long gvol = (long)nf_[0] * ny_ * nf_[2];
     cudaStream_t st = ctx.stream();
-    // values read once, fine grid written once (plus the permutation)
-    ProfScope ps(ctx, PS_SPREAD, (double)nvol * (8.0 * pts_.M + 8.0 * gvol) + 4.0 * pts_.M);
+    // lattice values read once (half of them when the others are conjugates), the
+    // kept fine grid written once, permutation and corners of the folded points
+    // read; the folded values and the fixed-point grid in between do not count
+    const double read = (double)pts_.ntheta * (herm ? pts_.half : pts_.lat);
+    ProfScope ps(ctx, PS_SPREAD, (double)nvol * (8.0 * read + 8.0 * gvol) + 6.0 * pts_.Mh);
     // two 32-bit fixed-point accumulators per cell (real and imaginary parts)
     // per volume, a footprint count per cell and the bucketed point order (16
     // bits per point)
@@ -1592,7 +1596,10 @@ void NufftPlan::spread(Context &ctx, const float2 *c, int nvol, float2 *grid, Pt
 void NufftPlan::interp(Context &ctx, const float2 *grid, int nvol, float2 *c, PtMode mode, int keep) {
     GridCfg g = make_cfg(dim_, nf_, bs_, nb_, w_, beta_, ylo_, ny_);
     const long gvol = (long)nf_[0] * ny_ * nf_[2];
-    ProfScope ps(ctx, PS_INTERP, (double)nvol * (8.0 * pts_.M + 8.0 * gvol) + 4.0 * pts_.M);
+    // the kept fine grid and the points' permutation and corners read once, the
+    // stored lattice values written once
+    const double written = (double)pts_.ntheta * keep;
+    ProfScope ps(ctx, PS_INTERP, (double)nvol * (8.0 * written + 8.0 * gvol) + 6.0 * pts_.Mh);
     const size_t tile_bytes = (size_t)g.td[0] * g.td[1] * g.td[2] * sizeof(float2);
     const Direct2D dir{dim_ == 2 && pts_.nrep == pts_.ntheta ? 1 : 0, 0, keep};
     if (!dir.on) vals_.ensure((long)nvol * pts_.Mh, ctx.stream());
