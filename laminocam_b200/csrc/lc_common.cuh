@@ -69,9 +69,11 @@ void note_kernel_launch();
 // the direct predecessor wrote is complete before a CTA starts.
 // Under stream capture the launches are plain: graphs with programmatic edges
 // were slower to replay (a 2D solve of 30 iterations 2.43 -> 2.88 ms).
-// A^T A of 1 x 255^2: 20.7 -> 19.0 us in a row, 31.9 -> 28.0 us alone; 8 x
-// 1023^2: 282 -> 273 us; 31 x 360 x 363, tilted: 176 -> 166 us; 29 x 721 x 721:
-// 531 -> 529 us (thousands of CTAs per pass: little to overlap).
+// A^T A, passes in a row, plain -> chained: 1 x 255^2 21.0 -> 19.0 us (runs of
+// one build differ by 3 %), 8 x 1023^2 280.7 -> 272.5 us, 31 x 360 x 363 tilted
+// 176.4 -> 167.7 us, 29 x 721 x 721 539.8 -> 536.3 us (thousands of CTAs per
+// pass: little to overlap).  The first pass on a fresh input, which the host's
+// work bounds, shows no difference (62 to 66 us for 1 x 255^2 either way).
 __device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

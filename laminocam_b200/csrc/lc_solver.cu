@@ -546,9 +546,10 @@ __device__ __forceinline__ void for_quads(const Tiles &tl, const Dims &dm, F &&b
 // is taken as c, everywhere else outside the volume as 0.  j and i are uniform
 // over the warp and the row's padding is zero, so only a row's first and last
 // voxel need a test; the tests per voxel and axis had the kernel at 65 % of its
-// issue slots and 56 % of its integer pipe.  (100 outer iterations on 29 x 721 x
-// 721, with the same for the padding of the projections: 109.1 -> 107.5 ms.)
-// The caller's factor takes the 0.25 (exact).
+// issue slots and 56 % of its integer pipe.  The gain is small, the arrays bound
+// the kernels: 20 outer iterations on 29 x 721 x 721 took 28.81 ms with the tests
+// and 28.69 ms without, where runs of one build differ by 0.1 ms.  The caller's
+// factor takes the 0.25 (exact).
 __device__ __forceinline__ Quad lap4(const float *__restrict__ x, long idx, int i, int j, int k0, const Dims &dm,
                                      const Quad &c, Quad m2k, Quad p2k) {
     const int sj = dm.p3, si = dm.n2 * dm.p3;
